@@ -242,7 +242,10 @@ int steps_gpu_batch_get(int k, double *x, double *v, double *F);
 
 /* Fixes the mixed-precision kernel shape: threads per block (64/128/256),
  * i-particles per thread (1/2/4) and j-range split (0 = automatic). Tile size
- * is threads*ipt. Returns STEPS_E_ARG for an unsupported shape. */
+ * is threads*ipt. Returns STEPS_E_ARG for an unsupported shape. A shape or
+ * variant (steps_gpu_set_kernel_variant) set explicitly is used as given;
+ * without one, and after steps_gpu_autotune, R^3 calls for the forces of all
+ * particles run a kernel that evaluates each pair once for both particles. */
 int steps_gpu_set_tuning(int threads, int ipt, int jsplit);
 
 /* R^3 mixed-precision pair loop: 0 = scalar FP32 instructions, 1 = packed
@@ -275,7 +278,10 @@ int steps_gpu_set_precision_guard(double ratio);
  * fastest; writes threads, ipt, variant to out[3]. Each candidate is first
  * timed on a strided sample of the range's i tiles against all j, 24 waves
  * of work (after one untimed launch); the three best are timed again on 96
- * waves (or the whole range when it is smaller). Leaves no resident forces. */
+ * waves (or the whole range when it is smaller). R^3 calls over all particles
+ * run the kernel that evaluates each pair once, faster than any of these
+ * shapes: nothing is timed for them, and out is the shape that other calls
+ * use. Leaves no resident forces. */
 int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out);
 
 /* Number of kernels this library has launched since init. */

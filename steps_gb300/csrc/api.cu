@@ -224,6 +224,28 @@ Tables device_tables(const KParams &kp)
     return t;
 }
 
+// Whether a mixed call for particles id_min .. id_min + ni - 1 of n can
+// evaluate each pair once.
+static bool sym_call(const KParams &kp, int n, int id_min, int ni)
+{
+    return id_min == 0 && ni == n && sym_supported(kp, n);
+}
+
+void mixed_dispatch(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,
+                    int id_min, int ni, double *F, bool reuse_order)
+{
+    Ctx &c = g_ctx;
+    if (c.shape.sym && !c.tune_sample && sym_call(kp, n, id_min, ni)) {
+        try {
+            forces_sym(kp, tb, x, m64, eps64, n, F, reuse_order);
+            return;
+        } catch (const Error &e) {
+            if (e.code != STEPS_E_NOMEM) throw;
+        }
+    }
+    forces_mixed(kp, tb, x, m64, eps64, n, id_min, ni, F, reuse_order);
+}
+
 void compute_forces(const steps_params *p, int precision, int id_min, int id_max, bool reuse_order)
 {
     Ctx &c = g_ctx;
@@ -249,8 +271,8 @@ void compute_forces(const steps_params *p, int precision, int id_min, int id_max
     if (precision == STEPS_FP64)
         forces_fp64(kp, tb, c.x.as<double>(), c.n, id_min, ni, F);
     else
-        forces_mixed(kp, tb, c.x.as<double>(), c.m64.as<double>(), c.eps64.as<double>(), c.n, id_min, ni, F,
-                     reuse_order);
+        mixed_dispatch(kp, tb, c.x.as<double>(), c.m64.as<double>(), c.eps64.as<double>(), c.n, id_min, ni, F,
+                       reuse_order);
     c.F_lo = id_min;
     c.F_ni = ni;
     c.F_valid = id_min == 0 && ni == c.n;
@@ -554,6 +576,7 @@ int steps_gpu_set_tuning(int threads, int ipt, int jsplit)
         g_ctx.shape.ipt = ipt;
         g_ctx.shape.jsplit = jsplit;
         g_ctx.shape_fixed = true;
+        g_ctx.shape.sym = false;
     });
 }
 
@@ -563,9 +586,28 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
         require_init();
         Ctx &c = g_ctx;
         static const int shapes[][2] = {{64, 1}, {64, 2}, {64, 4}, {128, 1}, {128, 2}, {128, 4}, {256, 1}, {256, 2}};
+        KParams kp = derive_params(p);
+        if (sym_call(kp, c.n, id_min, id_max - id_min + 1)) {
+            // The pairwise kernel is at least as fast as every one-sided shape
+            // at the sizes it takes (within 3 % at n = 16,384, 1.2 times from
+            // 32,768 on, 1.35 times at 2^20), so nothing is timed; one
+            // evaluation sizes the buffers.
+            const bool keep_sym = c.shape.sym;
+            c.shape.sym = true;
+            try {
+                compute_forces(p, STEPS_MIXED, id_min, id_max, false);
+            } catch (...) {
+                c.shape.sym = keep_sym;
+                throw;
+            }
+            c.shape_fixed = true;
+            c.F_ni = 0;
+            c.F_valid = false;
+            if (out) { out[0] = c.shape.threads; out[1] = c.shape.ipt; out[2] = c.shape.variant; }
+            return;
+        }
         Shape keep = c.shape;
         Shape bestS = keep;
-        KParams kp = derive_params(p);
         // R^3: the scalar and packed pair loops as well; T^3 with a table: the
         // one-i-per-lane and quad-lane kernels.
         const int nvar = kp.topology == STEPS_R3                          ? R3_VARIANTS
@@ -635,6 +677,7 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
             const double sc = score(scored[k].second, 96, false);
             if (sc < best) { best = sc; bestS = scored[k].second; }
         }
+        bestS.sym = true;  // calls over all particles
         c.shape = bestS;
         c.shape_fixed = true;
         if (out) { out[0] = bestS.threads; out[1] = bestS.ipt; out[2] = bestS.variant; }
@@ -665,6 +708,7 @@ int steps_gpu_set_kernel_variant(int variant)
             fail(STEPS_E_ARG, "kernel variant must be 0 (scalar), 1 (packed FP32x2), 2 or 3 (packed, 768 or 1024 "
                               "threads per SM) or 4 (packed, bulk-copy pipeline); for T3, 1 selects quad lanes");
         g_ctx.shape.variant = variant;
+        g_ctx.shape.sym = false;
     });
 }
 

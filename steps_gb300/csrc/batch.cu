@@ -395,7 +395,7 @@ void plain_steps(Batch &b, const KParams &kp, int precision, int nsteps, double 
         double *x = b.x.as<double>() + 3 * o, *F = b.F.as<double>() + 3 * o;
         const double *m = b.m64.as<double>() + o, *e = b.eps64.as<double>() + o;
         if (precision == STEPS_FP64) fail(STEPS_E_ARG, "batch: FP64 ensembles are not supported");
-        forces_mixed(kp, tb, x, m, e, b.n[k], 0, b.n[k], F, false);
+        mixed_dispatch(kp, tb, x, m, e, b.n[k], 0, b.n[k], F, false);
     };
     for (int k = 0; k < b.count; k++) force(k);
     for (int s = 0; s < nsteps; s++) {

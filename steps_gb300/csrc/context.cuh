@@ -82,7 +82,7 @@ Tables device_tables(const KParams &kp);
 // Padding ids: j padding and i padding differ so a padded i never meets a padded j.
 constexpr uint32_t PAD_J = 0xffffffffu, PAD_I = 0xfffffffeu;
 void build_tiles(TileSet &ts, const double *x, const double *m64, const double *eps64, int lo, int count, int T,
-                 bool reuse, cudaStream_t st, unsigned long long *bbox_scratch, uint32_t pad_id);
+                 bool reuse, cudaStream_t st, unsigned long long *bbox_scratch, uint32_t pad_id, int round_tiles = 1);
 // Stable LSD radix sort of (keys, vals) on key bits [lo_bit, 64).
 void sort_pairs(TileSet &ts, int n, cudaStream_t st, int lo_bit = 0);
 int morton_sort_bits(int n);
@@ -99,6 +99,21 @@ void forces_fp64(const KParams &kp, const Tables &tb, const double *x, int n, in
 struct MixedLaunch;
 void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64,
                   int n, int id_min, int ni, double *F, bool reuse_order);
+// pair_sym.cu: full-range mixed forces with every pair of particles evaluated
+// once. sym_supported: the calls it takes.
+// From SYM_MIN_N on: below, the one-sided kernels with small tiles fill the GPU
+// better (n = 8,192: 70 us against 99; 12,000: 124 against 127; 16,384: 181
+// against 186, tuned; 24,000: 328 against 312, pair kernel and reduction).
+constexpr int SYM_MIN_N = 16384;
+constexpr int SYM_NP4_N = 65536;  // from here on rows of 256 particles instead of 128
+constexpr long long SYM_PARTIAL_BYTES = 16LL << 30;  // FP64 partial sums of both sides at most
+bool sym_supported(const KParams &kp, int n);
+// A mixed call: the pairwise kernel where the call and the shape allow it, else (or where its partial sums do not fit
+// in device memory) the one-sided kernels.
+void mixed_dispatch(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,
+                    int id_min, int ni, double *F, bool reuse_order);
+void forces_sym(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,
+                double *F, bool reuse_order);
 bool shape_supported(int threads, int ipt);
 bool shape_supported_for(const KParams &kp, int threads, int ipt);
 

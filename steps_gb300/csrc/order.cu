@@ -216,13 +216,14 @@ void sort_pairs(TileSet &ts, int n, cudaStream_t st, int lo_bit)
 // Orders particles [lo, lo+count) of the AoS FP64 array x along a Morton curve
 // (unless reuse is set and an order already exists) and (re)builds the tiles.
 void build_tiles(TileSet &ts, const double *x, const double *m64, const double *eps64, int lo, int count, int T,
-                 bool reuse, cudaStream_t st, unsigned long long *bbox_scratch, uint32_t pad_id)
+                 bool reuse, cudaStream_t st, unsigned long long *bbox_scratch, uint32_t pad_id, int round_tiles)
 {
     if (count <= 0) fail(STEPS_E_ARG, "empty particle set");
     bool same = ts.ordered && ts.lo == lo && ts.count == count;
     ts.T = T;
     ts.ntiles = div_up(count, T);
-    size_t padded = (size_t)ts.ntiles * T;
+    const int nbuilt = div_up(ts.ntiles, round_tiles) * round_tiles;  // the rest are empty (all padding)
+    size_t padded = (size_t)nbuilt * T;
     if (!(reuse && same)) {
         for (int b = 0; b < 2; b++) {
             ts.keys[b].ensure<unsigned long long>(count);
@@ -243,12 +244,12 @@ void build_tiles(TileSet &ts, const double *x, const double *m64, const double *
     }
     ts.pack.ensure<float4>(padded);
     ts.eps.ensure<float>(padded);
-    ts.meta.ensure<float4>(2 * (size_t)ts.ntiles);
+    ts.meta.ensure<float4>(2 * (size_t)nbuilt);
     ts.idx.ensure<uint32_t>(padded);
     ts.resid.ensure<float4>(padded);
     ts.soa.ensure<float4>(padded);
     ts.sub.ensure<float4>(2 * (padded / SUBTILE));
-    k_tile_build<<<ts.ntiles, TB_THREADS, 0, st>>>(x, m64, eps64, ts.perm(), (long long)lo + count, count, T,
+    k_tile_build<<<nbuilt, TB_THREADS, 0, st>>>(x, m64, eps64, ts.perm(), (long long)lo + count, count, T,
                                                    ts.pack.as<float4>(),
                                                    ts.eps.as<float>(), ts.meta.as<float4>(), ts.idx.as<uint32_t>(),
                                                    pad_id, ts.resid.as<float4>(), ts.soa.as<float>(), nullptr,
