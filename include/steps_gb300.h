@@ -244,8 +244,10 @@ int steps_gpu_batch_get(int k, double *x, double *v, double *F);
  * i-particles per thread (1/2/4) and j-range split (0 = automatic). Tile size
  * is threads*ipt. Returns STEPS_E_ARG for an unsupported shape. A shape or
  * variant (steps_gpu_set_kernel_variant) set explicitly is used as given;
- * without one, and after steps_gpu_autotune, R^3 calls for the forces of all
- * particles run a kernel that evaluates each pair once for both particles. */
+ * without one, and after steps_gpu_autotune, calls for the forces of all
+ * particles (from 16,384 on in R^3, 4,096 on in the periodic topologies) run a
+ * kernel that evaluates each pair once for both particles; with a correction
+ * table only if the table is odd in the separation, as the builders' are. */
 int steps_gpu_set_tuning(int threads, int ipt, int jsplit);
 
 /* R^3 mixed-precision pair loop: 0 = scalar FP32 instructions, 1 = packed
@@ -278,10 +280,10 @@ int steps_gpu_set_precision_guard(double ratio);
  * fastest; writes threads, ipt, variant to out[3]. Each candidate is first
  * timed on a strided sample of the range's i tiles against all j, 24 waves
  * of work (after one untimed launch); the three best are timed again on 96
- * waves (or the whole range when it is smaller). R^3 calls over all particles
- * run the kernel that evaluates each pair once, faster than any of these
- * shapes: nothing is timed for them, and out is the shape that other calls
- * use. Leaves no resident forces. */
+ * waves (or the whole range when it is smaller). Calls over all particles that
+ * run the kernel evaluating each pair once (steps_gpu_set_tuning) are faster
+ * than with any of these shapes: nothing is timed for them, and out is the
+ * shape that other calls use. Leaves no resident forces. */
 int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out);
 
 /* Number of kernels this library has launched since init. */

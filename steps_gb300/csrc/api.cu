@@ -226,16 +226,16 @@ Tables device_tables(const KParams &kp)
 
 // Whether a mixed call for particles id_min .. id_min + ni - 1 of n can
 // evaluate each pair once.
-static bool sym_call(const KParams &kp, int n, int id_min, int ni)
+static bool sym_call(const KParams &kp, const Tables &tb, int n, int id_min, int ni)
 {
-    return id_min == 0 && ni == n && sym_supported(kp, n);
+    return id_min == 0 && ni == n && sym_supported(kp, tb, n);
 }
 
 void mixed_dispatch(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,
                     int id_min, int ni, double *F, bool reuse_order)
 {
     Ctx &c = g_ctx;
-    if (c.shape.sym && !c.tune_sample && sym_call(kp, n, id_min, ni)) {
+    if (c.shape.sym && !c.tune_sample && sym_call(kp, tb, n, id_min, ni)) {
         try {
             forces_sym(kp, tb, x, m64, eps64, n, F, reuse_order);
             return;
@@ -587,10 +587,11 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
         Ctx &c = g_ctx;
         static const int shapes[][2] = {{64, 1}, {64, 2}, {64, 4}, {128, 1}, {128, 2}, {128, 4}, {256, 1}, {256, 2}};
         KParams kp = derive_params(p);
-        if (sym_call(kp, c.n, id_min, id_max - id_min + 1)) {
-            // The pairwise kernel is at least as fast as every one-sided shape
-            // at the sizes it takes (within 3 % at n = 16,384, 1.2 times from
-            // 32,768 on, 1.35 times at 2^20), so nothing is timed; one
+        if (sym_call(kp, device_tables(kp), c.n, id_min, id_max - id_min + 1)) {
+            // The pairwise kernels are at least as fast as every one-sided
+            // shape at the sizes they take (R^3: within 3 % at n = 16,384, 1.2
+            // times from 32,768 on, 1.35 times at 2^20; periodic: 1.1-1.8 times
+            // at 5,000, about twice from 8,000 on), so nothing is timed; one
             // evaluation sizes the buffers.
             const bool keep_sym = c.shape.sym;
             c.shape.sym = true;

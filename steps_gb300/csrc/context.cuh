@@ -43,6 +43,10 @@ struct Ctx {
     DevBuf s1rec;              // S1xR2 table records: whole CIC stencils or TSC z triplets
     long long s1rec_version = -1;
     int s1rec_order = -1;             // layout of s1rec: CIC (2) or TSC (4)
+    // Whether the correction tables are odd in the separation (pair_box.cu),
+    // for the version last looked at.
+    long long t3_odd_version = -1, s1_odd_version = -1;
+    bool t3_odd = false, s1_odd = false;
     DevBuf s1r2;
     int nrho = 0, nz = 0;
     long long s1r2_version = 0;
@@ -105,9 +109,11 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
 // better (n = 8,192: 70 us against 99; 12,000: 124 against 127; 16,384: 181
 // against 186, tuned; 24,000: 328 against 312, pair kernel and reduction).
 constexpr int SYM_MIN_N = 16384;
+constexpr int BOX_MIN_N = 4096;  // periodic topologies (n = 3,000 / 5,000, one-sided tuned -> pairwise, us: trilinear 189 /
+                               // 393 -> 175 / 251, CIC 66 / 143 -> 101 / 119, images 95 / 179 -> 99 / 132)
 constexpr int SYM_NP4_N = 65536;  // from here on rows of 256 particles instead of 128
 constexpr long long SYM_PARTIAL_BYTES = 16LL << 30;  // FP64 partial sums of both sides at most
-bool sym_supported(const KParams &kp, int n);
+bool sym_supported(const KParams &kp, const Tables &tb, int n);
 // A mixed call: the pairwise kernel where the call and the shape allow it, else (or where its partial sums do not fit
 // in device memory) the one-sided kernels.
 void mixed_dispatch(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,

@@ -258,6 +258,12 @@ __device__ __forceinline__ f2 f2_sub(f2 a, f2 b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
 {
     f2 r;
@@ -368,6 +374,8 @@ using EnsembleFn = void (*)(EnsembleArgs);
 
 }  // namespace mixed
 
+// pair_mixed.cu: the periods, tolerances and precision guard of the arguments.
+void period_args(mixed::MixedArgs &a, const KParams &kp);
 // pair_t3.cu: T^3 kernel for a shape (dynamic shared memory returned) and its
 // table arguments (FP32 table copy, grid geometry).
 // variant 0: one i per lane (optionally with the shared-memory window);

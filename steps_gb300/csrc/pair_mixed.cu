@@ -451,6 +451,33 @@ bool shape_supported_for(const KParams &kp, int threads, int ipt)
     return select_kernel(kp, threads, ipt) != nullptr;
 }
 
+// Periods, tolerances and the precision guard; no tables.
+void period_args(mixed::MixedArgs &a, const KParams &kp)
+{
+    Ctx &c = ctx();
+    a.L = (float)kp.L;
+    a.halfL = (float)kp.halfL;
+    a.cutL = (float)kp.cutL;
+    a.cut_tol = (float)(kp.cutL * 1e-5);
+    a.L_lo = (float)(kp.L - (double)a.L);
+    a.halfL_lo = (float)(kp.halfL - (double)a.halfL);
+    a.wrap_tol = (float)(kp.halfL * 1e-5);
+    a.guard2 = c.shape.guard * c.shape.guard;
+    a.emax = kp.emax;
+    a.nearest = kp.topology == STEPS_S1R2 && kp.is_periodic < 2;
+    a.t3f = nullptr;
+    a.ng = 0;
+    a.ih = a.u0 = 0.0f;
+    a.wcap = 0;
+    a.halo = a.ext = 0;
+    a.t3r = nullptr;
+    a.t3rz = nullptr;
+    a.s1tab = nullptr;
+    a.s1rec = nullptr;
+    a.nrho = a.nz = 0;
+    a.irho = a.iz = a.rho_max = 0.0f;
+}
+
 bool mixed_supported(const KParams &kp) { return select_kernel(kp, 128, 2) != nullptr; }
 
 void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64,
@@ -543,27 +570,7 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
     a.items = nullptr;
     a.part_stride = (size_t)nit * T * 3;
     a.part = c.partial.ensure<double>((size_t)S * a.part_stride);
-    a.L = (float)kp.L;
-    a.halfL = (float)kp.halfL;
-    a.cutL = (float)kp.cutL;
-    a.cut_tol = (float)(kp.cutL * 1e-5);
-    a.L_lo = (float)(kp.L - (double)a.L);
-    a.halfL_lo = (float)(kp.halfL - (double)a.halfL);
-    a.wrap_tol = (float)(kp.halfL * 1e-5);
-    a.guard2 = c.shape.guard * c.shape.guard;
-    a.emax = kp.emax;
-    a.nearest = kp.topology == STEPS_S1R2 && kp.is_periodic < 2;
-    a.t3f = nullptr;
-    a.ng = 0;
-    a.ih = a.u0 = 0.0f;
-    a.wcap = 0;
-    a.halo = a.ext = 0;
-    a.t3r = nullptr;
-    a.t3rz = nullptr;
-    a.s1tab = nullptr;
-    a.s1rec = nullptr;
-    a.nrho = a.nz = 0;
-    a.irho = a.iz = a.rho_max = 0.0f;
+    period_args(a, kp);
     if (kp.topology == STEPS_T3) t3_args(a, kp, tb, st);
     if (s1tab) s1tab_args(a, kp, tb, st);
 

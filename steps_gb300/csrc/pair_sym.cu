@@ -37,7 +37,8 @@
 // of the one-sided kernels and take the double-float path, after the far ones.
 //
 // Measured (GB300, clustered compactified sets, pair kernel, one-sided packed
-// kernel -> this one): n = 32,768: 628 (tuned 525) -> 421 us; 262,144: 28.3 -> 19.4 ms; 2^20: 404 -> 297 ms, the FMA pipe 77 % busy.
+// kernel -> this one): n = 32,768: 628 (tuned 525) -> 421 us; 262,144:
+// 28.3 -> 19.4 ms; 2^20: 404 -> 297 ms, the FMA pipe 77 % busy.
 // Further warps per SM (fewer registers, NP = 2), scalar instead of packed
 // sums, other unrollings and a single rotated sum instead of two all measured
 // within 3 % or slower: the FMA pipe with its operand reads is the limit.
@@ -46,41 +47,14 @@
 #include "common.cuh"
 #include "context.cuh"
 #include "mixed.cuh"
+#include "sym.cuh"
 
 
-#ifndef SYM_BLK
-#define SYM_BLK 4
-#define SYM_UNR 8
-#define SYM_DUP 0
-#define SYM_ROT 0
-#define SYM_NP 4
-#define SYM_ORD 0
-#endif
 namespace steps {
 
 namespace {
 
 using namespace mixed;
-
-constexpr int SYM_T = 128;                 // particles per tile
-constexpr int SYM_WARPS = 4;               // per block; each works on its own
-constexpr int SYM_THREADS = 32 * SYM_WARPS;
-constexpr int SYM_HALF = SYM_T / 2;
-constexpr int SYM_NSUB = SYM_T / SUBTILE;  // 8 sub-tile boxes per tile
-
-struct SymArgs {
-    const float4 *pack, *resid, *meta, *sub;
-    const float *eps;
-    const uint32_t *idx;
-    int njt;     // tiles that hold particles (arrays are padded to whole rows)
-    int nrows;
-    int G, C;    // rows per group, j chunks per group
-    int nitems;  // groups x C
-    unsigned *counter;
-    double *pi, *pj;  // partial sums [C][3][npad] and [groups][3][npad]
-    size_t npad;
-    float guard2;
-};
 
 // A warp's shared memory; NP packed i pairs per lane.
 template <int NP>
@@ -126,24 +100,6 @@ __device__ __forceinline__ void quad_box(const float4 *sub, float4 &c, float4 &h
 // normal FP32 number: boxes further apart or nearer than these bounds take the
 // near path, whose products start with a mass.
 constexpr float SYM_FAR2_MAX = 1e23f, SYM_GAP2_MIN = 1e-24f;
-
-// The j slabs cover only the particles that a group can meet: slab A starts
-// at particle start(A) = 64 A G NP and holds npad - start(A).
-// Returns the particles in the slabs before A (NP is even, so start is linear in A).
-template <int NP>
-__host__ __device__ inline size_t sym_slab(int A, int G, size_t npad)
-{
-    return (size_t)A * npad - (size_t)SYM_HALF * NP * G * ((size_t)A * (A - 1) / 2);
-}
-
-// Adds to the j-side partial sum of this (group, chunk), which only this lane
-// writes: the first row stores, later ones add in the memory system (in
-// program order, so the sum is deterministic).
-__device__ __forceinline__ void add_j(double *o, double v, bool first)
-{
-    if (first) *o = v;
-    else asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(v) : "memory");
-}
 
 // d_O + e_O = centre of tile J less the centre of half tile H's tile, exactly.
 __device__ __forceinline__ void frame_offset(const SymArgs &a, int J, int H, float *dO, float *eO)
@@ -258,7 +214,7 @@ __global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_sym_r3(SymArgs
 
         // this group's j slab: the padded particles from its first tile on
         const size_t jlo = (size_t)first * SYM_T, jlen = a.npad - jlo;
-        double *pj = a.pj + 3 * sym_slab<NP>(A, a.G, a.npad);
+        double *pj = a.pj + 3 * sym_slab(A, a.step, 1, a.npad);
 
         for (int r = row0; r < row1; r++) {
             int H0 = r * NP;  // this row's half tiles: H0 .. H0 + NP - 1
@@ -360,7 +316,7 @@ __global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_sym_r3(SymArgs
                         f2_unpack(JZ, v[2][0], v[2][1]);
 #pragma unroll
                         for (int c = 0; c < 3; c++)
-                            add_j(oj + c * jlen + g * 32, (double)(v[c][0] + v[c][1]), firstrow);
+                            add_slab(oj + c * jlen + g * 32, (double)(v[c][0] + v[c][1]), firstrow);
                     }
                 }
 #pragma unroll
@@ -396,7 +352,7 @@ __global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_sym_r3(SymArgs
                         }
                         if (both)
 #pragma unroll
-                            for (int c = 0; c < 3; c++) add_j(oj + c * jlen + g * 32, jd[c], firstrow);
+                            for (int c = 0; c < 3; c++) add_slab(oj + c * jlen + g * 32, jd[c], firstrow);
                     }
             }
 #pragma unroll
@@ -414,9 +370,8 @@ __global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_sym_r3(SymArgs
 // slab in order, and the first adds the 8 sums in order. The sums of a few
 // hundred slabs are latency-bound with one thread per component at small n.
 constexpr int RED_PARTS = 8;
-template <int NP>
 __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__restrict__ pi,
-                                                               const double *__restrict__ pj, int C, int G, size_t npad,
+                                                               const double *__restrict__ pj, SymPlan p,
                                                                const uint32_t *__restrict__ perm, int count,
                                                                const double *__restrict__ x, Background bg,
                                                                double *__restrict__ F)
@@ -426,17 +381,17 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__r
     const int q = blockIdx.x * 32 + lane;  // < npad
     double f[3] = {0.0, 0.0, 0.0};
 #pragma unroll 4
-    for (int s = w; s < C; s += RED_PARTS)
+    for (int s = w; s < p.C; s += RED_PARTS)
 #pragma unroll
-        for (int c = 0; c < 3; c++) f[c] += pi[((size_t)s * 3 + c) * npad + q];
-    const int r = q / (SYM_HALF * NP);  // met from the i side by the rows before its own
-    const int ng = r > 0 ? (r - 1) / G + 1 : 0;
+        for (int c = 0; c < 3; c++) f[c] += pi[((size_t)s * 3 + c) * p.npad + q];
+    const int r = q / p.gran;  // met from the i side by the granules before its own
+    const int ng = r > 0 ? (r - 1) / p.G + 1 : 0;
 #pragma unroll 4
     for (int A = w; A < ng; A += RED_PARTS) {
-        const size_t start = (size_t)A * SYM_HALF * NP * G, len = npad - start;
-        const double *p = pj + 3 * sym_slab<NP>(A, G, npad) + (q - start);
+        const size_t start = p.tri ? (size_t)A * p.step : 0, len = p.npad - start;
+        const double *o = pj + 3 * sym_slab(A, p.step, p.tri, p.npad) + (q - start);
 #pragma unroll
-        for (int c = 0; c < 3; c++) f[c] -= p[c * len];
+        for (int c = 0; c < 3; c++) f[c] -= o[c * len];
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) part[w][c][lane] = f[c];
@@ -455,14 +410,23 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__r
 
 }  // namespace
 
+// Groups and chunks of a plan whose granules are set: at most 256 groups and
+// 128 chunks, the slabs within the partial-sum budget.
+bool sym_split(SymPlan &p)
+{
+    const long long slabs = std::max<long long>(SYM_PARTIAL_BYTES / (24 * (long long)p.npad), 1);
+    p.G = div_up(p.nrows, (int)std::min<long long>(256, slabs));
+    p.tri = (long long)p.gran * p.G % SYM_T == 0;
+    p.step = p.gran * p.G;
+    p.groups = div_up(p.nrows, p.G);
+    p.C = (int)std::min<long long>(std::min(128, p.ntiles), std::max<long long>(slabs / 2, 1));
+    p.doubles = 3 * ((size_t)p.C * p.npad + sym_slab(p.groups, p.step, p.tri, p.npad));
+    return slabs >= 160;
+}
+
 namespace {
 
-struct SymPlan {
-    int NP, ntiles, nrows, G, groups, C;
-    size_t npad, doubles;  // padded particles; partial sums
-};
-
-// Row width, rows per group and chunks per group for n particles. Narrow rows
+// Row width for n particles. Narrow rows
 // give small sets enough warps, wide ones amortise the rotation (pair kernel,
 // NP = 1 / 2 / 4: n = 32,768 439 / 421 / 456 us; 65,536 1566 / 1445 / 1400 us).
 bool sym_plan(int n, SymPlan &p)
@@ -471,17 +435,12 @@ bool sym_plan(int n, SymPlan &p)
     p.ntiles = div_up(n, SYM_T);
     p.nrows = div_up(2 * p.ntiles, p.NP);
     p.npad = (size_t)div_up(p.nrows * p.NP, 2) * SYM_T;
-    const long long slabs = SYM_PARTIAL_BYTES / (24 * (long long)p.npad);
-    p.G = div_up(p.nrows, (int)std::min<long long>(256, std::max<long long>(slabs, 1)));
-    p.groups = div_up(p.nrows, p.G);
-    p.C = (int)std::min<long long>(std::min(128, p.ntiles), std::max<long long>(slabs / 2, 1));
-    const size_t jslabs = p.NP == 4 ? sym_slab<4>(p.groups, p.G, p.npad) : sym_slab<2>(p.groups, p.G, p.npad);
-    p.doubles = 3 * ((size_t)p.C * p.npad + jslabs);
-    return slabs >= 160;
+    p.gran = SYM_HALF * p.NP;
+    return sym_split(p);
 }
 
 template <int NP>
-void sym_launch(const SymPlan &p, SymArgs a, const Background &bg, const double *x, int n, double *F)
+void sym_launch(const SymArgs &a)
 {
     Ctx &c = ctx();
     int occ = 0;
@@ -489,18 +448,15 @@ void sym_launch(const SymPlan &p, SymArgs a, const Background &bg, const double 
     const int grid = std::min(div_up(a.nitems, SYM_WARPS), c.nsm * std::max(occ, 1));
     k_sym_r3<NP><<<grid, SYM_THREADS, 0, c.stream>>>(a);
     note_launch("k_sym_r3");
-    STEPS_CUDA(cudaEventRecord(c.phase[2], c.stream));
-    k_sym_reduce<NP><<<div_up(n, 32), 32 * RED_PARTS, 0, c.stream>>>(a.pi, a.pj, a.C, a.G, a.npad, c.tj.perm(), n, x,
-                                                                    bg, F);
-    note_launch("k_sym_reduce");
 }
 
 }  // namespace
 
-bool sym_supported(const KParams &kp, int n)
+bool sym_supported(const KParams &kp, const Tables &tb, int n)
 {
     SymPlan p;
-    return kp.topology == STEPS_R3 && n >= SYM_MIN_N && sym_plan(n, p);
+    if (kp.topology == STEPS_R3) return n >= SYM_MIN_N && sym_plan(n, p);
+    return n >= BOX_MIN_N && box_plan(n, p) && box_supported(kp, tb);
 }
 
 void forces_sym(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,
@@ -509,7 +465,8 @@ void forces_sym(const KParams &kp, const Tables &tb, const double *x, const doub
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
     SymPlan p;
-    if (!sym_plan(n, p)) fail(STEPS_E_ARG, "pairwise kernel: too many particles");
+    const bool box = kp.topology != STEPS_R3;
+    if (!(box ? box_plan(n, p) : sym_plan(n, p))) fail(STEPS_E_ARG, "pairwise kernel: too many particles");
     STEPS_CUDA(cudaEventRecord(c.phase[0], st));
     build_tiles(c.tj, x, m64, eps64, 0, n, SYM_T, reuse_order, st, c.bbox.ensure<unsigned long long>(8), PAD_J,
                 (int)(p.npad / SYM_T));
@@ -525,6 +482,8 @@ void forces_sym(const KParams &kp, const Tables &tb, const double *x, const doub
     a.nrows = p.nrows;
     a.G = p.G;
     a.C = p.C;
+    a.step = p.step;
+    a.tri = p.tri;
     a.nitems = p.groups * p.C;
     a.counter = c.counter.ensure<unsigned>(4);
     a.npad = p.npad;
@@ -533,8 +492,12 @@ void forces_sym(const KParams &kp, const Tables &tb, const double *x, const doub
     a.guard2 = c.shape.guard * c.shape.guard;
     STEPS_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), st));
     const Background bg = background_of(kp, tb);
-    if (p.NP == 4) sym_launch<4>(p, a, bg, x, n, F);
-    else sym_launch<2>(p, a, bg, x, n, F);
+    if (box) box_launch(kp, tb, a);
+    else if (p.NP == 4) sym_launch<4>(a);
+    else sym_launch<2>(a);
+    STEPS_CUDA(cudaEventRecord(c.phase[2], st));
+    k_sym_reduce<<<div_up(n, 32), 32 * RED_PARTS, 0, st>>>(a.pi, a.pj, p, c.tj.perm(), n, x, bg, F);
+    note_launch("k_sym_reduce");
     STEPS_CUDA(cudaEventRecord(c.phase[3], st));
     c.phase_valid = true;
     c.last_pairs = (double)n * (double)n;

@@ -1,5 +1,7 @@
 """The pairwise kernels (each pair of particles evaluated once, added to both)
 against the FP64 kernels, at the edges of tiles, rows, row widths and groups."""
+import math
+
 import numpy as np
 import pytest
 
@@ -87,3 +89,82 @@ def test_r3_kdk_and_choice(fresh):
         out.append(fresh.state())
     assert err_stats(out[0][2], out[1][2])["p99"] < MIXED_P99
     assert np.abs(out[0][0] - out[1][0]).max() < 1e-6
+
+
+# ---- periodic topologies ------------------------------------------------------
+
+L3, LZ = 100.0, 200.0
+
+
+def periodic(eng, kind, n, seed=1):
+    """A workload set and parameters; the table, if the kind has one, is built."""
+    if kind.startswith("t3"):
+        ps = W.t3_clumpy(n, L3, seed)
+        order = int(kind[2:])
+        if order:
+            eng.build_table_t3(31, L3, 2.0 / L3, 2.0, 5.0 * 2.0 * math.pi / L3, 3.0, 6.0)
+        return ps, S.params(S.T3, is_periodic=2 if order else 1, L=L3, rsim=L3 / 2, ewald_order=order or 2)
+    ps = W.s1r2_cylindrical(n, LZ, 600.0, seed)
+    if kind == "s1tab2" or kind == "s1tab4":
+        eng.build_table_s1r2(432, 64, 2.25 * 600.0, LZ, 0.787875 / LZ, 4, 10)
+        return ps, S.params(S.S1R2, is_periodic=2, L=LZ, rsim=600.0, s1r2_images=0, ewald_order=int(kind[-1]))
+    return ps, S.params(S.S1R2, is_periodic=int(kind[2:]), L=LZ, rsim=600.0, s1r2_images=1)
+
+
+KINDS = ["t30", "t32", "t34", "s11", "s12", "s115", "s1tab2", "s1tab4"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [4096, 4127, 8192, 8193, 16385, 33000])
+def test_periodic_sizes(fresh, kind, n):
+    """Taken from n = 4,096 on; groups are one block up to 8,192, two up to 16,384, whole tiles above."""
+    ps, p = periodic(fresh, kind, n)
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(ps.x, p, S.MIXED)
+    for lo in (0, n - 700):
+        st = err_stats(F[lo:lo + 700], fresh.forces(ps.x, p, S.FP64, lo, lo + 699))
+        assert st["p99"] < MIXED_P99, (kind, n, lo, st)
+    assert np.array_equal(F, fresh.forces(ps.x, p, S.MIXED))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_periodic_hard_decisions(fresh, kind):
+    """Pairs within a few FP32 ulps of half a period along each axis and of the image cut: the image is the FP64
+    kernel's. (Pairs at half a period to the last FP64 bits, below the 48 bits that mixed positions hold, may fall
+    either way in every mixed kernel: they are computed beside the others and not compared.)"""
+    n = 6000
+    ps, p = periodic(fresh, kind, n, seed=7)
+    rng = np.random.default_rng(3)
+    x = ps.x.copy()
+    period = L3 if kind.startswith("t3") else LZ
+    axes = (0, 1, 2) if kind.startswith("t3") else (2,)
+    dist = [period / 2] + ([2.6 * LZ % LZ] if kind == "s12" else [])
+    a, b = np.arange(0, 2000, 2), np.arange(1, 2000, 2)
+    for k, (i, j) in enumerate(zip(a, b)):
+        ax, d = axes[k % len(axes)], dist[k // 3 % len(dist)]
+        x[j] = x[i] + rng.normal(0.0, 0.5, 3)
+        x[j, ax] = x[i, ax] + d * (1.0 + (k % 7 - 3) * 2.0 ** -23)
+        x[j] = x[j] if not kind.startswith("t3") else x[j] % period
+        x[j, 2] %= period
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(x, p, S.MIXED)
+    resolved = np.repeat(np.arange(1000) % 7 != 3, 2)
+    st = err_stats(F[:2000][resolved], fresh.forces(x, p, S.FP64, 0, 1999)[resolved])
+    assert st["p99"] < MIXED_P99, st
+    assert st["max"] < 1e-3, st  # a flipped image moves a particle's force by per cents
+
+
+@pytest.mark.parametrize("topology", ["t32", "s1tab2"])
+def test_tables_that_are_not_odd(fresh, topology):
+    """A table without the symmetry of an Ewald correction is used as given (by the one-sided kernels)."""
+    n = 5000
+    ps, p = periodic(fresh, topology, n)
+    rng = np.random.default_rng(2)
+    if topology == "t32":
+        fresh.set_table_t3(rng.normal(0.0, 1e-4, 3 * 31 ** 3), 31)
+    else:
+        fresh.set_table_s1r2(rng.normal(0.0, 1e-6, 2 * 432 * 64), 432, 64)
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(ps.x, p, S.MIXED)
+    fresh.set_tuning(128, 2, 0)  # the default shape, one-sided
+    assert np.array_equal(F, fresh.forces(ps.x, p, S.MIXED))
