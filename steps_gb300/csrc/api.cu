@@ -361,7 +361,7 @@ int steps_gpu_shutdown(void)
         cudaSetDevice(c.device);
         cudaStreamSynchronize(c.stream);
         batch_release();
-        DevBuf *bufs[] = {&c.m64, &c.eps64, &c.x, &c.v, &c.F, &c.pack64, &c.partial, &c.bbox, &c.counter,
+        DevBuf *bufs[] = {&c.m64, &c.eps64, &c.x, &c.v, &c.F, &c.pack64, &c.epsf64, &c.partial, &c.bbox, &c.counter,
                           &c.status, &c.flush, &c.peaks, &c.t3, &c.t3f, &c.t3r, &c.s1r2, &c.s1f, &c.s1rec,
                           &c.radial, &c.kstatus};
         for (DevBuf *b : bufs) b->release();

@@ -249,6 +249,54 @@ __device__ __forceinline__ double rsqrt_fp64(double x)
     return fma(y * e, p, y);
 }
 
+// r^-3 of a pair known to be outside its softening support, from r^2, on as few
+// FP64 instructions as it takes (4). The FP64 pipe, 1/64 of the FP32 rate,
+// bounds the FP64 kernels, so what other pipes can do exactly or accurately
+// enough is moved there. With the MUFU seed y ~ r^-1 and e = 1 - r^2 y^2,
+//   r^-3 = y^3 (1 + 3 e / 2 + 15 e^2 / 8 + O(e^3)),  |e| < 2^-20.9:
+//   * r^2 and y change format by integer instructions (the conversions run on
+//     the FP64 pipe);
+//   * y^2 is exact in 48 bits, an integer product;
+//   * 15 e^2 / 8 < 2^-40.8 is needed to 2^-13 of itself: FP32.
+// b2: an FP32 upper bound of the squared support. False, with w untouched,
+// where r^2 may lie inside it or outside the FP32 range: the caller then takes
+// softening_fp64. Against the 10 instructions of rsqrt_fp64, its conversions
+// and cube, and 3 for the comparison: R^3 at n = 32,768, one-sided 43.7 -> 31.1
+// ms (with 6 instructions here).
+__device__ __forceinline__ double widen_fp32(int bits)  // a normal, positive float
+{
+    return __hiloint2double((bits >> 3) + (896 << 20), bits << 29);
+}
+
+__device__ __forceinline__ bool far_r3_fp64(double r2, float b2, double &w)
+{
+    const int hi = __double2hiint(r2), lo = __double2loint(r2);
+    const float f = __int_as_float((int)__funnelshift_l((unsigned)lo, (unsigned)hi - (896u << 20), 3));  // truncated
+    if (!((unsigned)hi - (897u << 20) < (253u << 20) && f > b2)) return false;
+    const int yb = __float_as_int(rsqrt_mufu(f));
+    const double y = widen_fp32(yb);
+    // y^2 = M^2 2^(2 E) with a 24-bit M: M^2 has 47 or 48 bits
+    const unsigned m = ((unsigned)yb & 0x7fffffu) | 0x800000u;
+    const unsigned long long mm = (unsigned long long)m * m;
+    const int top = (int)(mm >> 47);
+    const long long ex = 2 * ((yb >> 23) - 127) + top + 1022;
+    const double q = __longlong_as_double((long long)(mm << (6 - top)) + (ex << 52));
+    const double e = fma(-r2, q, 1.0), y3 = q * y;
+    const int eh = max(__double2hiint(e) & 0x7fffffff, 897 << 20);
+    const float ef = __int_as_float((eh - (896 << 20)) << 3);
+    const double s2 = widen_fp32(__float_as_int(1.875f * ef * ef));  // 2^-127 where it underflows
+    w = fma(y3, fma(1.5, e, s2), y3);
+    return true;
+}
+
+// FP32 bound for far_r3_fp64 of the support (ei + ej)^2, from softening lengths
+// rounded up to FP32 (1e-5 covers the FP32 sum and square and f's truncation).
+__device__ __forceinline__ float support2_fp32(float ei, float ej)
+{
+    const float b = ei + ej;
+    return b * b * 1.00001f;
+}
+
 // Cubic-spline softened force coefficient w(r, beta) for r < beta (the
 // r >= beta branch is 1/r^3). StePS/src/forces.cc:52-87,
 // StePS/src/forces_cuda.cu:466-519, written in u = r / beta:
@@ -271,6 +319,16 @@ __device__ __forceinline__ double softening_fp64(double r2, double beta)
         return y * y * y;
     }
     return spline_inner_fp64(sqrt(r2), beta);
+}
+
+// Softened weight w(r^2) of a pair; beta() gives its softening support, read
+// only where it matters.
+template <class Beta>
+__device__ __forceinline__ double weight_fp64(double r2, float b2, Beta beta)
+{
+    double w;
+    if (!far_r3_fp64(r2, b2, w)) w = softening_fp64(r2, beta());
+    return w;
 }
 
 __device__ __forceinline__ float spline_inner_f32(float r2, float beta)

@@ -24,6 +24,7 @@ struct Ctx {
     bool F_valid = false;            // F holds full-range forces of the current x
     int F_lo = 0, F_ni = 0;          // range F currently holds
     DevBuf pack64;                   // FP64 kernel j stream: (x, y, z, m) per particle
+    DevBuf epsf64;                   // its softening lengths rounded up to FP32
     DevBuf partial;                  // per-j-chunk partial forces (FP64)
     DevBuf bbox, counter, status, flush, peaks;
     DevBuf kstatus;                  // int written by kernels whose bounded waits give up
@@ -46,7 +47,7 @@ struct Ctx {
     // Whether the correction tables are odd in the separation (pair_box.cu),
     // for the version last looked at.
     long long t3_odd_version = -1, s1_odd_version = -1;
-    bool t3_odd = false, s1_odd = false;
+    double t3_odd = 1.0, s1_odd = 1.0;  // largest asymmetry over the largest entry
     DevBuf s1r2;
     int nrho = 0, nz = 0;
     long long s1r2_version = 0;
@@ -109,6 +110,7 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
 // better (n = 8,192: 70 us against 99; 12,000: 124 against 127; 16,384: 181
 // against 186, tuned; 24,000: 328 against 312, pair kernel and reduction).
 constexpr int SYM_MIN_N = 16384;
+constexpr int SYM_FP64_MIN_N = 512;
 constexpr int BOX_MIN_N = 4096;  // periodic topologies (n = 3,000 / 5,000, one-sided tuned -> pairwise, us: trilinear 189 /
                                // 393 -> 175 / 251, CIC 66 / 143 -> 101 / 119, images 95 / 179 -> 99 / 132)
 constexpr int SYM_NP4_N = 65536;  // from here on rows of 256 particles instead of 128

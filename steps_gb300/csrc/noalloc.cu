@@ -112,12 +112,13 @@ __global__ void __launch_bounds__(NA_THREADS)
                       int n, int id_min, int ni, int jchunk, double *__restrict__ part)
 {
     __shared__ double4_16a sp[NA_THREADS];
-    __shared__ double se[NA_THREADS];
+    __shared__ float se[NA_THREADS];  // rounded up
     const int t = threadIdx.x;
     const int li = blockIdx.x * NA_THREADS + t;
     const bool active = li < ni;
     const size_t i = (size_t)id_min + (active ? li : 0);
-    const double xi = x[3 * i], yi = x[3 * i + 1], zi = x[3 * i + 2], ei = eps[i];
+    const double xi = x[3 * i], yi = x[3 * i + 1], zi = x[3 * i + 2];
+    const float ei = __double2float_ru(eps[i]);
     const int j0 = blockIdx.y * jchunk;
     const int j1 = min(n, j0 + jchunk);
     double ax = 0, ay = 0, az = 0;
@@ -127,13 +128,14 @@ __global__ void __launch_bounds__(NA_THREADS)
         if (t < cnt) {
             const size_t j = (size_t)jb + t;
             sp[t] = make_double4_16a(x[3 * j], x[3 * j + 1], x[3 * j + 2], m[j]);
-            se[t] = eps[j];
+            se[t] = __double2float_ru(eps[j]);
         }
         __syncthreads();
         for (int jj = 0; jj < cnt; ++jj) {
             const double4_16a q = sp[jj];
             const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-            const double w = q.w * softening_fp64(dx * dx + dy * dy + dz * dz, ei + se[jj]);
+            const double w = q.w * weight_fp64(dx * dx + dy * dy + dz * dz, support2_fp32(ei, se[jj]),
+                                               [&] { return eps[i] + eps[(size_t)jb + jj]; });
             ax = fma(w, dx, ax);
             ay = fma(w, dy, ay);
             az = fma(w, dz, az);

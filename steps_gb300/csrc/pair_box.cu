@@ -610,10 +610,8 @@ __global__ void k_table_parity(const double *__restrict__ t, long long ncell, in
     atomicMax(&out[1], bb);
 }
 
-// Odd to 1e-9 of the largest entry: 1/60 of the FP32 rounding of the entries
-// that the mixed kernels read. The builders' tables are odd exactly or to
-// rounding; any other table takes the one-sided kernels.
-static bool table_odd(const double *t, long long ncell, int nz)
+// Largest asymmetry of a table over its largest entry (NaN: not comparable).
+static double asymmetry(const double *t, long long ncell, int nz)
 {
     Ctx &c = ctx();
     unsigned long long *d = c.bbox.ensure<unsigned long long>(8), h[2];
@@ -624,7 +622,26 @@ static bool table_odd(const double *t, long long ncell, int nz)
     STEPS_CUDA(cudaStreamSynchronize(c.stream));
     double v[2];
     memcpy(v, h, sizeof v);
-    return v[0] <= 1e-9 * v[1];  // false for NaN
+    return v[0] == 0.0 ? v[0] * v[1] : v[0] / v[1];
+}
+
+// The correction table of a call is odd in the separation to tol of its largest
+// entry. Looked at once per table.
+static bool table_odd(const KParams &kp, const Tables &tb, double tol)
+{
+    Ctx &c = ctx();
+    if (kp.topology == STEPS_T3) {
+        if (c.t3_odd_version != c.t3_version) {
+            c.t3_odd = asymmetry(tb.t3, (long long)tb.t3_ng * tb.t3_ng * tb.t3_ng, 0);
+            c.t3_odd_version = c.t3_version;
+        }
+        return c.t3_odd <= tol;
+    }
+    if (c.s1_odd_version != c.s1r2_version) {
+        c.s1_odd = asymmetry(tb.s1r2, (long long)tb.nrho * tb.nz, tb.nz);
+        c.s1_odd_version = c.s1r2_version;
+    }
+    return c.s1_odd <= tol;
 }
 
 static int box_kind(const KParams &kp)
@@ -644,22 +661,18 @@ bool box_supported(const KParams &kp, const Tables &tb)
     if (kind < 0) return false;
     if (kind == B_S1_IMG) return kp.emax < 64;  // 7 bits per image number
     if (kind == B_S1_NEAR) return kp.L < 1e11 && kp.rsim < 1e11;  // r^-3 stays a normal FP32 number
-    if (kind == B_T3_LIN || kind == B_T3_CUB) {
-        if (c.shape.t3_cells > 0) return false;  // the caller asked for the shared-memory window
-        if (c.t3_odd_version != c.t3_version) {
-            c.t3_odd = table_odd(tb.t3, (long long)tb.t3_ng * tb.t3_ng * tb.t3_ng, 0);
-            c.t3_odd_version = c.t3_version;
-        }
-        return c.t3_odd;
-    }
-    if (kind == B_S1_CIC || kind == B_S1_TSC) {
-        if (c.s1_odd_version != c.s1r2_version) {
-            c.s1_odd = table_odd(tb.s1r2, (long long)tb.nrho * tb.nz, tb.nz);
-            c.s1_odd_version = c.s1r2_version;
-        }
-        return c.s1_odd;
-    }
-    return true;
+    if ((kind == B_T3_LIN || kind == B_T3_CUB) && c.shape.t3_cells > 0)
+        return false;  // the caller asked for the shared-memory window
+    // Odd to 1e-9 of the largest entry: 1/60 of the FP32 rounding of the entries
+    // that the mixed kernels read. The builders' tables are odd exactly or to
+    // rounding; any other table takes the one-sided kernels.
+    return kind == B_T3_NEAR || table_odd(kp, tb, 1e-9);
+}
+
+bool fp64_odd(const KParams &kp, const Tables &tb)
+{
+    const int kind = kp.topology == STEPS_R3 ? B_S1_NEAR : box_kind(kp);
+    return kind >= 0 && (kind == B_S1_NEAR || kind == B_S1_IMG || kind == B_T3_NEAR || table_odd(kp, tb, 1e-16));
 }
 
 // Granules are the 32-particle i blocks: groups of one or two of them for sets

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__r
     for (int v = 1; v < RED_PARTS; v++)
 #pragma unroll
         for (int c = 0; c < 3; c++) f[c] += part[v][c][lane];
-    long long o = perm[q];
+    long long o = perm ? (long long)perm[q] : q;
     STEPS_CHECK_IDX(o, count, CK_OUTPUT);
     add_background(bg, x + 3 * (size_t)o, f);
 #pragma unroll
@@ -412,11 +412,11 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__r
 
 // Groups and chunks of a plan whose granules are set: at most 256 groups and
 // 128 chunks, the slabs within the partial-sum budget.
-bool sym_split(SymPlan &p)
+bool sym_split(SymPlan &p, int tile)
 {
     const long long slabs = std::max<long long>(SYM_PARTIAL_BYTES / (24 * (long long)p.npad), 1);
     p.G = div_up(p.nrows, (int)std::min<long long>(256, slabs));
-    p.tri = (long long)p.gran * p.G % SYM_T == 0;
+    p.tri = (long long)p.gran * p.G % tile == 0;
     p.step = p.gran * p.G;
     p.groups = div_up(p.nrows, p.G);
     p.C = (int)std::min<long long>(std::min(128, p.ntiles), std::max<long long>(slabs / 2, 1));
@@ -451,6 +451,14 @@ void sym_launch(const SymArgs &a)
 }
 
 }  // namespace
+
+void sym_reduce(const SymPlan &p, const double *part, const uint32_t *perm, int n, const double *x, const Background &bg,
+                double *F)
+{
+    k_sym_reduce<<<div_up(n, 32), 32 * RED_PARTS, 0, ctx().stream>>>(part, part + 3 * (size_t)p.C * p.npad, p, perm, n, x,
+                                                                    bg, F);
+    note_launch("k_sym_reduce");
+}
 
 bool sym_supported(const KParams &kp, const Tables &tb, int n)
 {
@@ -496,8 +504,7 @@ void forces_sym(const KParams &kp, const Tables &tb, const double *x, const doub
     else if (p.NP == 4) sym_launch<4>(a);
     else sym_launch<2>(a);
     STEPS_CUDA(cudaEventRecord(c.phase[2], st));
-    k_sym_reduce<<<div_up(n, 32), 32 * RED_PARTS, 0, st>>>(a.pi, a.pj, p, c.tj.perm(), n, x, bg, F);
-    note_launch("k_sym_reduce");
+    sym_reduce(p, a.pi, c.tj.perm(), n, x, bg, F);
     STEPS_CUDA(cudaEventRecord(c.phase[3], st));
     c.phase_valid = true;
     c.last_pairs = (double)n * (double)n;

@@ -55,11 +55,18 @@ __device__ __forceinline__ void add_slab(double *o, double v, bool first)
     else asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(v) : "memory");
 }
 
-bool sym_split(SymPlan &p);  // pair_sym.cu
+// pair_sym.cu: groups and chunks of a plan whose granules are set (groups that
+// are whole tiles of `tile` particles get triangular slabs); the reduction of
+// the slabs into F (perm: curve order to the caller's, NULL: the same).
+bool sym_split(SymPlan &p, int tile = SYM_T);
+void sym_reduce(const SymPlan &p, const double *part, const uint32_t *perm, int n, const double *x, const Background &bg,
+                double *F);
 bool box_plan(int n, SymPlan &p);
 // pair_box.cu: whether a periodic call can take the pairwise kernel (its kind,
 // and a correction table that is odd in the separation), and the launch.
 bool box_supported(const KParams &kp, const Tables &tb);
+// The same for FP64: a table that is odd to the last bits, or none.
+bool fp64_odd(const KParams &kp, const Tables &tb);
 void box_launch(const KParams &kp, const Tables &tb, const SymArgs &s);
 
 }  // namespace steps

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import steps_gb300 as S
-from helpers import err_stats
+from helpers import err_stats, rel_err
 from steps_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -168,3 +168,39 @@ def test_tables_that_are_not_odd(fresh, topology):
     F = fresh.forces(ps.x, p, S.MIXED)
     fresh.set_tuning(128, 2, 0)  # the default shape, one-sided
     assert np.array_equal(F, fresh.forces(ps.x, p, S.MIXED))
+
+
+# ---- FP64 -----------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("kind", ["r3", "t30", "t32", "t34", "s11", "s12", "s1tab2"])
+@pytest.mark.parametrize("n", [511, 512, 543, 2000, 8193])
+def test_fp64_sizes(fresh, kind, n):
+    """All particles (each pair once, from n = 512 on) against the two halves (one-sided): the difference is the order
+    of the sums, 1e-16 times a few. Groups hold two rows from 8,193 on."""
+    if kind == "r3":
+        ps, p = W.r3_compactified(n, 480.0, seed=n, displace=True), S.params(S.R3, cosmology=1, comoving=1, mius=1e-3)
+    else:
+        ps, p = periodic(fresh, kind, n)
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(ps.x, p, S.FP64)
+    half = np.concatenate([fresh.forces(ps.x, p, S.FP64, 0, n // 2), fresh.forces(ps.x, p, S.FP64, n // 2 + 1, n - 1)])
+    assert rel_err(F, half).max() < 1e-11
+    assert np.median(rel_err(F, half)) < 1e-14
+    assert np.array_equal(F, fresh.forces(ps.x, p, S.FP64))
+
+
+def test_fp64_softened_and_far_units(fresh, port):
+    """Pairs inside and at the edge of the spline, a coincident pair, and lengths where r^2 leaves the FP32 range."""
+    import pyoracle as O
+    from helpers import port_params
+    rng = np.random.default_rng(5)
+    x = rng.normal(0, 0.05, (600, 3))
+    x[1] = x[0]
+    x[3] = x[2] + np.array([0.2, 0, 0])
+    m, eps = rng.uniform(0.5, 2.0, 600), np.full(600, 0.1)
+    for scale in (1.0, 1e-12, 1e15):
+        fresh.set_particles(m, eps * scale)
+        F = fresh.forces(x * scale, S.params(S.R3), S.FP64)
+        Fo = port.forces(port.system(0, m, eps * scale, port_params(O)), x * scale)
+        assert rel_err(F, Fo).max() < 1e-11, scale
