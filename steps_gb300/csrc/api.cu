@@ -601,10 +601,10 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
                 c.shape.sym = keep_sym;
                 throw;
             }
-            c.shape_fixed = true;
             c.F_ni = 0;
             c.F_valid = false;
-            if (out) { out[0] = c.shape.threads; out[1] = c.shape.ipt; out[2] = c.shape.variant; }
+            const Shape other = c.shape_fixed ? c.shape : auto_shape(kp, c.n, c.n);
+            if (out) { out[0] = other.threads; out[1] = other.ipt; out[2] = other.variant; }
             return;
         }
         Shape keep = c.shape;
@@ -710,6 +710,7 @@ int steps_gpu_set_kernel_variant(int variant)
                               "threads per SM) or 4 (packed, bulk-copy pipeline); for T3, 1 selects quad lanes");
         g_ctx.shape.variant = variant;
         g_ctx.shape.sym = false;
+        g_ctx.shape_fixed = true;
     });
 }
 

@@ -81,7 +81,7 @@ struct TileSet {
     const uint32_t *perm() const { return vals[perm_sel].as<uint32_t>(); }
 };
 
-// Mixed-kernel launch shape.
+// Mixed-kernel launch shape (one-sided kernels; auto_shape where the caller set none).
 struct Shape {
     int threads = 128;
     int ipt = 2;

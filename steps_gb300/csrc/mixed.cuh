@@ -374,7 +374,9 @@ using EnsembleFn = void (*)(EnsembleArgs);
 
 }  // namespace mixed
 
-// pair_mixed.cu: the periods, tolerances and precision guard of the arguments.
+// pair_mixed.cu: the one-sided kernel shape where the caller chose none; the
+// periods, tolerances and precision guard of the arguments.
+Shape auto_shape(const KParams &kp, int ni, int n);
 void period_args(mixed::MixedArgs &a, const KParams &kp);
 // pair_t3.cu: T^3 kernel for a shape (dynamic shared memory returned) and its
 // table arguments (FP32 table copy, grid geometry).

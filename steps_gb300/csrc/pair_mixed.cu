@@ -386,17 +386,38 @@ __global__ void __launch_bounds__(BLOCK, KIND == K_R3 && IPT == 1 ? 1024 / BLOCK
     }
 }
 
-// Sum the chunk partials in chunk order, add the background term and scatter
-// from curve order back to the caller's order F[3*(orig - id_min) + k].
-__global__ void k_reduce_mixed(const double *__restrict__ part, int S, size_t stride, const uint32_t *__restrict__ perm,
-                               int count, int id_min, const double *__restrict__ x, Background bg,
-                               double *__restrict__ F)
+// Sum the chunk partials, add the background term and scatter from curve order
+// back to the caller's order F[3*(orig - id_min) + k]. A block takes 32
+// particles; its 8 warps sum every 8th chunk in order and the first adds the 8
+// sums in order: with one thread per particle a short range against many
+// chunks waits for one load after the other (1,000 i, 977 chunks: 221 us).
+constexpr int RED_PARTS = 8;
+__global__ void __launch_bounds__(32 * RED_PARTS) k_reduce_mixed(const double *__restrict__ part, int S, size_t stride,
+                                                                 const uint32_t *__restrict__ perm, int count,
+                                                                 int id_min, const double *__restrict__ x,
+                                                                 Background bg, double *__restrict__ F)
 {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= count) return;
+    __shared__ double sh[RED_PARTS][96];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int q0 = blockIdx.x * 32;
+    // the 96 components of the block's particles lie in a row: lane l sums
+    // components l, 32 + l, 64 + l (rows are padded to whole tiles)
     double f[3] = {0, 0, 0};
-    for (int s = 0; s < S; s++)
-        for (int k = 0; k < 3; k++) f[k] += part[(size_t)s * stride + 3 * (size_t)q + k];
+#pragma unroll 4
+    for (int s = w; s < S; s += RED_PARTS)
+#pragma unroll
+        for (int k = 0; k < 3; k++) f[k] += part[(size_t)s * stride + 3 * (size_t)q0 + 32 * k + lane];
+#pragma unroll
+    for (int k = 0; k < 3; k++) sh[w][32 * k + lane] = f[k];
+    __syncthreads();
+    const int q = q0 + lane;
+    if (w != 0 || q >= count) return;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        f[k] = sh[0][3 * lane + k];
+#pragma unroll
+        for (int v = 1; v < RED_PARTS; v++) f[k] += sh[v][3 * lane + k];
+    }
     uint32_t o = perm[q];
     long long row = (long long)o - id_min;
     STEPS_CHECK_IDX(row, count, CK_OUTPUT);
@@ -480,22 +501,50 @@ void period_args(mixed::MixedArgs &a, const KParams &kp)
 
 bool mixed_supported(const KParams &kp) { return select_kernel(kp, 128, 2) != nullptr; }
 
+// The one-sided kernel shape where the caller chose none, for ni particles
+// against n. R^3: small tiles give small calls enough items; from 2.5e7 pairs
+// on 256 x 1 at 1024 threads an SM, from 8e9 on 128 x 2 (measured, us, 128 x 2
+// scalar -> this: 2,000^2 160 -> 15, 3,001^2 151 -> 24, 3,000 x 30,000 189 ->
+// 89, 20,000 x 100,000 1424 -> 962, 66,667 x 200,003 7401 -> 5600). Periodic:
+// 64 x 1, whose smaller boxes send fewer pairs down the near path (33,333 x
+// 100,000, ms, 128 x 2 -> 64 x 1: trilinear 34.0 -> 29.3, images 17.8 -> 8.8,
+// nearest image 6.1 -> 3.7); from 1e9 pairs on 256 x 1 for the wide stencils,
+// which re-read the table less (tricubic 250 -> 192, CIC 13.2 -> 11.7).
+Shape auto_shape(const KParams &kp, int ni, int n)
+{
+    Shape s = ctx().shape;
+    const double pairs = (double)ni * (double)n;
+    if (kp.topology == STEPS_R3) {
+        s.threads = pairs < 2.5e7 ? 64 : pairs < 8e9 ? 256 : 128;
+        s.ipt = pairs < 8e9 ? 1 : 2;
+        s.variant = pairs < 2.5e7 || pairs >= 8e9 ? 1 : 3;
+        return s;
+    }
+    if (kp.topology == STEPS_T3 && s.t3_cells > 0) return s;  // the shared-memory window was chosen for 128 x 2
+    const bool s1tab = kp.topology == STEPS_S1R2 && kp.is_periodic >= 2 && !kp.s1r2_images;
+    const bool wide = kp.topology == STEPS_T3 ? kp.is_periodic >= 2 && kp.order == 4 : s1tab && kp.order != 0;
+    s.threads = wide && pairs >= 1e9 ? 256 : 64;
+    s.ipt = 1;
+    return s;
+}
+
 void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64,
                   int n, int id_min, int ni, double *F, bool reuse_order)
 {
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
-    const int threads = c.shape.threads, ipt = c.shape.ipt;
+    const Shape shape = c.shape_fixed || c.tune_sample > 0 ? c.shape : auto_shape(kp, ni, n);
+    const int threads = shape.threads, ipt = shape.ipt;
     const int T = threads * ipt;
     size_t dyn = 0;
     const bool s1tab = kp.topology == STEPS_S1R2 && kp.is_periodic >= 2 && !kp.s1r2_images;
-    const bool packed = kp.topology == STEPS_R3 && c.shape.variant >= 1;
+    const bool packed = kp.topology == STEPS_R3 && shape.variant >= 1;
     // T^3 reads the variant as 0 (one i per lane) or 1 (quad lanes); the R^3
     // pair loops 2-4 have no T^3 counterpart and mean 0 there.
-    KernelFn fn = kp.topology == STEPS_T3 ? t3_kernel(kp, threads, ipt, &dyn, c.shape.variant == 1 ? 1 : 0)
+    KernelFn fn = kp.topology == STEPS_T3 ? t3_kernel(kp, threads, ipt, &dyn, shape.variant == 1 ? 1 : 0)
                   : s1tab              ? s1tab_kernel(kp, threads, ipt)
-                  : packed             ? (c.shape.variant == 4 ? r3x2_pipe_kernel(threads, ipt)
-                                                               : r3x2_kernel(threads, ipt, false, r3x2_occ(c.shape.variant)))
+                  : packed             ? (shape.variant == 4 ? r3x2_pipe_kernel(threads, ipt)
+                                                               : r3x2_kernel(threads, ipt, false, r3x2_occ(shape.variant)))
                                        : select_kernel(kp, threads, ipt);
     if (!fn) fail(STEPS_E_ARG, "mixed precision: unsupported topology/mode or kernel shape");
 
@@ -516,16 +565,19 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
     if (occ < 1) occ = 1;
     const int resident = c.nsm * occ;
     const int nit = ti.ntiles, njt = c.tj.ntiles;
-    int S = c.shape.jsplit;
+    int S = shape.jsplit;
     // The FP64 chunk partials (S x N_i x 24 B) stay within 4 GiB.
     const long long smax = std::max(1LL, (4LL << 30) / ((long long)nit * T * 24));
     if (S <= 0) {
-        // Items of at most 64 and at least 4 j tiles, aiming at 16 or more
-        // waves of items over the persistent grid: long items balance badly
-        // (near-field tile pairs make their lengths uneven), very short ones
-        // pay the per-item set-up.
+        // Up to two waves of tile pairs over the persistent grid: one wave of
+        // items of equal length. Above, items of at most 64 j tiles, aiming at
+        // 48 or more waves: long items balance badly (near-field tile pairs
+        // make their lengths uneven). R^3, 256 x 1 (1024 threads an SM): 12,000
+        // x 12,000 103 us with 1-tile items, 110 with 2; 30,000 x 40,000 581 us
+        // with 2, 605 with 4; 128 x 2: 66,667 x 200,003 5.6 ms with 4, 5.9 with 16.
         const long long pairs = (long long)nit * njt;
-        const long long tpc = std::min(64LL, std::max(4LL, pairs / (16LL * resident)));
+        const long long tpc = pairs <= 2LL * resident ? (pairs + resident - 1) / resident
+                                                      : std::min(64LL, std::max(1LL, pairs / (48LL * resident)));
         S = (int)std::min<long long>(smax, (njt + tpc - 1) / tpc);
         if (S < 1) S = 1;
     }
@@ -578,7 +630,7 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
     a.stall_seq = c.stall_seq;
     c.stall_seq = -1;
     STEPS_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned), st));
-    const bool bounded_waits = packed && c.shape.variant == 4;
+    const bool bounded_waits = packed && shape.variant == 4;
     if (bounded_waits) STEPS_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int), st));
     int grid = resident < a.nitems ? resident : a.nitems;
     fn<<<grid, threads, dyn, st>>>(a);
@@ -592,7 +644,7 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
     }
     STEPS_CUDA(cudaEventRecord(c.phase[2], st));
     if (!sample) {
-        k_reduce_mixed<<<div_up(ni, 256), 256, 0, st>>>(a.part, S, a.part_stride, ti.perm(), ni, id_min, x,
+        k_reduce_mixed<<<div_up(ni, 32), 32 * RED_PARTS, 0, st>>>(a.part, S, a.part_stride, ti.perm(), ni, id_min, x,
                                                        background_of(kp, tb), F);
         note_launch("k_reduce_mixed");
     }

@@ -1,0 +1,51 @@
+"""The one-sided kernel shape and j split that are chosen when the caller set none, at the sizes where the choice
+changes, against the FP64 kernels."""
+import pytest
+
+import steps_gb300 as S
+from helpers import err_stats
+from steps_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def fresh(engine):
+    """The engine with no shape or variant chosen."""
+    engine.shutdown()
+    yield S.Engine(0)
+    engine.set_tuning(128, 2, 0)
+    engine.set_variant(0)
+
+
+# (n, first, count): one particle, one tile, below and above 2.5e7 and 8e9 pairs, short ranges against many particles
+RANGES = [(1, 0, 1), (64, 0, 63), (65, 1, 64), (5001, 0, 4990), (5011, 0, 5005), (100003, 5, 1), (100003, 50000, 33),
+          (120001, 20000, 66000), (120001, 0, 67500)]
+
+
+@pytest.mark.parametrize("n,lo,count", RANGES)
+def test_r3(fresh, n, lo, count):
+    ps = W.r3_compactified(n, 480.0, seed=n, displace=True)
+    fresh.set_particles(ps.m, ps.eps)
+    p = S.params(S.R3, cosmology=1, comoving=1, mius=1e-3)
+    F = fresh.forces(ps.x, p, S.MIXED, lo, lo + count - 1)
+    k = min(count, 500)
+    assert err_stats(F[-k:], fresh.forces(ps.x, p, S.FP64, lo + count - k, lo + count - 1))["p99"] < 1e-5
+
+
+@pytest.mark.parametrize("kind", ["t3", "tab0", "tab2", "img"])
+@pytest.mark.parametrize("n,lo,count", [(63, 0, 63), (4095, 0, 4095), (40000, 100, 24000), (40000, 100, 26000)])
+def test_periodic(fresh, kind, n, lo, count):
+    """Wide stencils change shape at 1e9 pairs; below n = 4,096 full ranges are one-sided."""
+    if kind == "t3":
+        ps, p = W.t3_clumpy(n, 100.0, 3), S.params(S.T3, is_periodic=2, L=100.0, rsim=50.0, ewald_order=4)
+        fresh.build_table_t3(31, 100.0, 0.02, 2.0, 0.3, 3.0, 6.0)
+    else:
+        ps = W.s1r2_cylindrical(n, 200.0, 600.0, 2)
+        p = S.params(S.S1R2, is_periodic=2, L=200.0, rsim=600.0, s1r2_images=int(kind == "img"),
+                     ewald_order=int(kind[-1]) if kind != "img" else 4)
+        fresh.build_table_s1r2(432, 64, 1350.0, 200.0, 0.787875 / 200.0, 4, 10)
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(ps.x, p, S.MIXED, lo, lo + count - 1)
+    k = min(count, 300)
+    assert err_stats(F[-k:], fresh.forces(ps.x, p, S.FP64, lo + count - k, lo + count - 1))["p99"] < 1e-5
