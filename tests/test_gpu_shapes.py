@@ -33,6 +33,23 @@ def test_r3(fresh, n, lo, count):
     assert err_stats(F[-k:], fresh.forces(ps.x, p, S.FP64, lo + count - k, lo + count - 1))["p99"] < 1e-5
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 512, 513, 1024, 1025, 2049, 4097, 8192, 8193, 16385, 32767, 32768, 32769])
+def test_ordering_sizes(fresh, n):
+    """Sets of up to 32,768 particles are ordered by one cluster of 1 to 8 blocks, 2, 4 or 8 particles a thread; with
+    coincident particles, one far outlier and (in y) all at one value."""
+    ps = W.r3_compactified(max(n, 2), 480.0, seed=n, displace=True)
+    x = ps.x[:n].copy()
+    x[:, 1] = 3.0
+    x[n // 2:n // 2 + 5] = x[0]
+    x[-1, 0] += 1e7
+    fresh.set_particles(ps.m[:n], ps.eps[:n])
+    p = S.params(S.R3)
+    F = fresh.forces(x, p, S.MIXED)
+    k = min(n, 400)
+    st = err_stats(F[:k], fresh.forces(x, p, S.FP64, 0, k - 1))
+    assert st["p99"] < 1e-5 or n == 1, st
+
+
 @pytest.mark.parametrize("kind", ["t3", "tab0", "tab2", "img"])
 @pytest.mark.parametrize("n,lo,count", [(63, 0, 63), (4095, 0, 4095), (40000, 100, 24000), (40000, 100, 26000)])
 def test_periodic(fresh, kind, n, lo, count):
