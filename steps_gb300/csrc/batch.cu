@@ -8,29 +8,26 @@
 // the sorted order; tiles never straddle two realisations (each realisation
 // is padded to a whole number of tiles).
 //
-// Work: a host-built list of items (i tile, j tile range, partial slot)
-// covering, for every realisation, its i tiles x j chunks; ordered by
-// realisation size, largest first, so the persistent kernel's atomic queue
-// schedules longest-processing-time first. The pair kernel is the packed
-// FP32x2 R^3 kernel in work-list mode; partial sums go to per-item slots and
-// a reduction adds each i tile's slots in order (deterministic).
-//
-// graph = 1: the whole run in ONE persistent kernel (k_ensemble, pair_r3x2.cu)
-// after a single ordering pass, captured into a CUDA graph and replayed:
-// (stage, item) tasks from one queue, a bounded wait per task on its
-// realisation's previous stage, the kicks, drift and tile rebuild done by the
-// block that finishes each tile. The tile shape, the j-chunk length and the
-// grid size are chosen by timing candidates first.
+// graph = 1: the whole run in ONE persistent kernel (ensemble.cu) after a
+// single ordering pass, captured into a CUDA graph and replayed: pair and finish
+// tasks of all realisations and stages from one queue, bounded waits between the
+// stages of a realisation. The row width and the size of the pair items are
+// chosen by timing candidates first.
 // graph = 2: the same run as a CUDA graph of per-phase kernels (per step:
 // kick+drift, re-order, re-tile, work-list force, reduction, kick).
+// Its work list of items (i tile, j tile range, partial slot), ordered by
+// realisation size, largest first, runs in the packed FP32x2 R^3 kernel in
+// work-list mode; a reduction adds each i tile's slots in order.
 // graph = 0: the same work as `count` separate single-realisation force calls
 // (and KDK kernels) per phase, for comparison.
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 #include <vector>
 
 #include "common.cuh"
 #include "context.cuh"
+#include "ensemble.cuh"
 #include "mixed.cuh"
 
 namespace steps {
@@ -52,13 +49,13 @@ struct Batch {
     long long graph_kernels = 0;
     int nmax = 0;  // largest realisation
     bool tuned = false;     // per-phase graph shape
-    bool ens_tuned = false; // persistent kernel shape, j-chunk length, grid
+    bool ens_tuned = false; // persistent kernel: row width and item size
     int threads_pp = 128, ipt_pp = 2;  // per-phase graph shape
-    int ens_threads = 128, ens_ipt = 2, ens_jmax = 256, ens_grid = 0;
-    double ens_frac = 1.0;
-    // persistent path: the second tile buffer, per-tile realisation, counters
-    DevBuf pack2, soa2, resid2, meta2, sub2;
-    DevBuf tile_rel, rel_ntiles, ens_ctl;
+    // persistent path
+    int ens_np = 2, ens_split = 16;
+    double ens_wait = 1.0;  // seconds a stage wait may last
+    int ens_tasks = 0;
+    DevBuf rels, tasks, ens_ctl;
     int stall_rel = -1;  // test hook for the next persistent run (one shot)
     cudaGraphExec_t exec = nullptr;
     int graph_steps = -1, graph_mode = 0;
@@ -149,9 +146,6 @@ void plan(Batch &b, int threads, int ipt, int jmax = 256)
     std::stable_sort(order.begin(), order.end(), [&](int a, int d) { return b.n[a] > b.n[d]; });
     std::vector<int4> items;
     std::vector<int2> tslot(b.ntiles);
-    std::vector<int> trel(b.ntiles);
-    for (int k = 0; k < b.count; k++)
-        for (int t = 0; t < nt[k]; t++) trel[tstart[k] + t] = k;
     for (int k : order) {
         const int S = div_up(nt[k], jmax);
         const int per = div_up(nt[k], S);
@@ -174,10 +168,6 @@ void plan(Batch &b, int threads, int ipt, int jmax = 256)
                                cudaMemcpyHostToDevice, c.stream));
     STEPS_CUDA(cudaMemcpyAsync(b.tslot.ensure<int2>(tslot.size()), tslot.data(), tslot.size() * sizeof(int2),
                                cudaMemcpyHostToDevice, c.stream));
-    STEPS_CUDA(cudaMemcpyAsync(b.tile_rel.ensure<int>(trel.size()), trel.data(), trel.size() * sizeof(int),
-                               cudaMemcpyHostToDevice, c.stream));
-    STEPS_CUDA(cudaMemcpyAsync(b.rel_ntiles.ensure<int>(nt.size()), nt.data(), nt.size() * sizeof(int),
-                               cudaMemcpyHostToDevice, c.stream));
     b.ts.pack.ensure<float4>(padded);
     b.ts.eps.ensure<float>(padded);
     b.ts.meta.ensure<float4>(2 * (size_t)b.ntiles);
@@ -185,12 +175,6 @@ void plan(Batch &b, int threads, int ipt, int jmax = 256)
     b.ts.resid.ensure<float4>(padded);
     b.ts.soa.ensure<float4>(padded);
     b.ts.sub.ensure<float4>(2 * (padded / SUBTILE));
-    b.pack2.ensure<float4>(padded);
-    b.soa2.ensure<float4>(padded);
-    b.resid2.ensure<float4>(padded);
-    b.meta2.ensure<float4>(2 * (size_t)b.ntiles);
-    b.sub2.ensure<float4>(2 * (padded / SUBTILE));
-    b.ens_ctl.ensure<unsigned>(1 + (size_t)b.ntiles + b.count);
     b.part.ensure<double>((size_t)b.nitems * T * 3);
     b.T = T;
     b.threads = threads;
@@ -203,9 +187,9 @@ void plan(Batch &b, int threads, int ipt, int jmax = 256)
     STEPS_CUDA(cudaStreamSynchronize(c.stream));
 }
 
-// Orders every realisation (one sort) and builds the tiles into the first
-// tile buffer (and, for the persistent kernel, the second one as well).
-void batch_order(Batch &b, bool both_buffers)
+// Orders every realisation (one sort) and builds the tiles; soa: with the SoA
+// copy that the work-list kernel reads.
+void batch_order(Batch &b, bool soa)
 {
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
@@ -223,13 +207,8 @@ void batch_order(Batch &b, bool both_buffers)
     sort_pairs(b.ts, b.ntot, st, std::max(0, 51 - std::min(51, morton_sort_bits(b.nmax))));
     tile_build_range(b.x.as<double>(), b.m64.as<double>(), b.eps64.as<double>(), b.ts.perm(), b.ntot, b.T,
                      b.ts.pack.as<float4>(), b.ts.eps.as<float>(), b.ts.meta.as<float4>(), b.ts.idx.as<uint32_t>(),
-                     PAD_J, b.ts.resid.as<float4>(), b.ts.soa.as<float>(), b.tdesc.as<int2>(), b.ntiles, st,
-                     b.ts.sub.as<float4>());
-    if (both_buffers)
-        tile_build_range(b.x.as<double>(), b.m64.as<double>(), b.eps64.as<double>(), b.ts.perm(), b.ntot, b.T,
-                         b.pack2.as<float4>(), b.ts.eps.as<float>(), b.meta2.as<float4>(), nullptr, PAD_J,
-                         b.resid2.as<float4>(), b.soa2.as<float>(), b.tdesc.as<int2>(), b.ntiles, st,
-                         b.sub2.as<float4>());
+                     PAD_J, b.ts.resid.as<float4>(), soa ? b.ts.soa.as<float>() : nullptr, b.tdesc.as<int2>(), b.ntiles,
+                     st, b.ts.sub.as<float4>());
 }
 
 // One batched force evaluation on the resident positions (stream-ordered; no
@@ -238,7 +217,7 @@ void batch_forces(Batch &b)
 {
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
-    batch_order(b, false);
+    batch_order(b, true);
 
     mixed::MixedArgs a{};
     a.stall_seq = -1;
@@ -268,107 +247,157 @@ void batch_forces(Batch &b)
 }
 
 // The whole run in one persistent kernel (stream-ordered, capturable): one
-// ordering pass that builds both tile buffers, the counters zeroed, then
-// k_ensemble over nsteps + 1 stages.
+// ordering pass, the counters zeroed, then k_ensemble over nsteps + 1 stages.
 void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
 {
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
-    batch_order(b, true);
+    batch_order(b, false);
     unsigned *ctl = b.ens_ctl.as<unsigned>();
-    STEPS_CUDA(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * (1 + (size_t)b.ntiles + b.count), st));
-    mixed::EnsembleArgs e{};
-    float4 *pk[2] = {b.ts.pack.as<float4>(), b.pack2.as<float4>()};
-    float *so[2] = {b.ts.soa.as<float>(), b.soa2.as<float>()};
-    float4 *re[2] = {b.ts.resid.as<float4>(), b.resid2.as<float4>()};
-    float4 *me[2] = {b.ts.meta.as<float4>(), b.meta2.as<float4>()};
-    float4 *su[2] = {b.ts.sub.as<float4>(), b.sub2.as<float4>()};
-    for (int k = 0; k < 2; k++) {
-        e.pack[k] = e.pack_w[k] = pk[k];
-        e.soa[k] = e.soa_w[k] = so[k];
-        e.resid[k] = e.resid_w[k] = re[k];
-        e.meta[k] = e.meta_w[k] = me[k];
-        e.sub[k] = e.sub_w[k] = su[k];
-    }
-    e.jeps = b.ts.eps.as<float>();
-    e.epsf_w = b.ts.eps.as<float>();
-    e.jidx = b.ts.idx.as<uint32_t>();
-    e.items = b.items.as<int4>();
-    e.nitems = b.nitems;
+    STEPS_CUDA(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * (1 + 2 * (size_t)b.count + b.ntiles), st));
+    EnsembleArgs e{};
+    e.rel = b.rels.as<EnsRel>();
+    e.tasks = b.tasks.as<int4>();
+    e.ntasks = b.ens_tasks;
     e.nstages = nsteps + 1;
-    e.tile_rel = b.tile_rel.as<int>();
-    e.tdesc = b.tdesc.as<int2>();
-    e.tslot = b.tslot.as<int2>();
-    e.rel_ntiles = b.rel_ntiles.as<int>();
-    e.perm = b.ts.perm();
+    e.nrel = b.count;
+    e.pack = b.ts.pack.as<float4>();
+    e.resid = b.ts.resid.as<float4>();
+    e.meta = b.ts.meta.as<float4>();
+    e.sub = b.ts.sub.as<float4>();
+    e.eps = b.ts.eps.as<float>();
+    e.idx = b.ts.idx.as<uint32_t>();
     e.part = b.part.as<double>();
     e.queue = ctl;
-    e.tile_cnt = ctl + 1;
-    e.rel_done = ctl + 1 + b.ntiles;
+    e.pair_done = ctl + 1;
+    e.fin_done = ctl + 1 + b.count;
+    e.tile_cnt = ctl + 1 + 2 * b.count;
     e.x = b.x.as<double>();
     e.v = b.v.as<double>();
     e.F = b.F.as<double>();
-    e.m64 = b.m64.as<double>();
-    e.eps64 = b.eps64.as<double>();
     e.h = h;
     e.guard2 = c.shape.guard * c.shape.guard;
+    e.n = b.ntot;
+    e.ntiles = b.ntiles;
     e.status = kernel_status_word();
     e.stall_rel = stall_rel;
-    e.ntiles = b.ntiles;
-    e.nslots = b.nitems;
-    e.nrel = b.count;
-    e.n = b.ntot;
-    mixed::EnsembleFn fn = ensemble_kernel(b.threads, b.ipt);
-    if (!fn) fail(STEPS_E_ARG, "batch: unsupported kernel shape");
-    fn<<<b.ens_grid, b.threads, 0, st>>>(e);
-    note_launch("k_ensemble");
+    e.wait_cycles = (long long)(b.ens_wait * (double)mixed::MBAR_WAIT_CYCLES);
+    ensemble_launch(b.ens_np, e, st);
     c.status_pending = true;
 }
 
-// Plans the work list for the persistent kernel's shape and sizes its grid:
-// `frac` of the blocks that fit on the GPU at once.
-void ensemble_plan(Batch &b, int threads, int ipt, int jmax, double frac)
+// Plans the persistent kernel for rows of 64 NP particles: tiles padded to whole
+// rows, and pair items so large that a stage has about `split` of them per
+// resident warp, at most `most` groups and chunks to a realisation (their number
+// sets the slabs).
+void ensemble_plan_most(Batch &b, int NP, int split, int most)
 {
     Ctx &c = ctx();
-    plan(b, threads, ipt, jmax);
-    mixed::EnsembleFn fn = ensemble_kernel(threads, ipt);
-    if (!fn) fail(STEPS_E_ARG, "batch: unsupported kernel shape");
-    int occ = 0;
-    STEPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, 0));
-    const int resident = c.nsm * std::max(occ, 1);
-    b.ens_grid = std::max(1, std::min(b.nitems, (int)(frac * resident)));
+    const int gran = SYM_HALF * NP, rt = NP / 2;  // particles and tiles of a row
+    std::vector<int2> desc;
+    std::vector<EnsRel> rel(b.count);
+    double units = 0.0, longest = 0.0;  // (row, tile) pairs, in all and of the largest item
+    for (int k = 0; k < b.count; k++) {
+        EnsRel &R = rel[k];
+        R = EnsRel{};
+        R.tile0 = (int)desc.size();
+        R.ntiles = div_up(b.n[k], SYM_T);
+        R.nrows = div_up(R.ntiles, rt);
+        R.gran = gran;
+        for (int t = 0; t < R.nrows * rt; t++)
+            desc.push_back(make_int2(b.off[k] + std::min(t * SYM_T, b.n[k]), std::max(0, std::min(SYM_T, b.n[k] - t * SYM_T))));
+        R.npad = (size_t)R.nrows * gran;
+        units += 0.5 * R.nrows * (double)R.ntiles;
+    }
+    const double warps = (double)c.nsm * ensemble_blocks(NP) * SYM_WARPS;
+    const double area = std::max(1.0, units / (warps * split));  // (row, tile) pairs of an item
+    std::vector<int> order(b.count);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b.n[x] > b.n[y]; });
+    size_t part = 0;
+    std::vector<int4> tasks;
+    for (int k : order) {
+        EnsRel &R = rel[k];
+        const double side = std::sqrt(area * rt);  // tiles
+        R.G = std::max(div_up(R.nrows, most), (int)std::lround(side / rt));
+        R.G = std::min(std::max(R.G, 1), R.nrows);
+        R.C = std::max(1, std::min(std::min(most, R.ntiles), (int)std::lround(R.ntiles / side)));
+        R.step = gran * R.G;
+        longest = std::max(longest, (double)R.G * div_up(R.ntiles, R.C));
+        const int groups = div_up(R.nrows, R.G);
+        R.npair = groups * R.C;
+        R.part = part;
+        part += 3 * ((size_t)R.C * R.npad + sym_slab(groups, R.step, 1, R.npad));
+        for (int A = 0; A < groups; A++)
+            for (int ch = 0; ch < R.C; ch++) tasks.push_back(make_int4(k, A, ch, 0));
+    }
+    for (int k : order)
+        for (int t = 0; t < 4 * rel[k].ntiles; t++) tasks.push_back(make_int4(k, t, 0, 1));
+    b.ens_tasks = (int)tasks.size();
+    b.ntiles = (int)desc.size();
+    b.T = SYM_T;
+    b.ens_np = NP;
+    b.ens_split = split;
+    // A stage wait lasts as long as a pair item at most, when all goes well: a
+    // warp evaluates 3e8 pairs a second beside its neighbours (bound: a second,
+    // or 8 times that).
+    b.ens_wait = std::max(1.0, 8.0 * longest * gran * SYM_T / 3e8);
+    const size_t padded = (size_t)b.ntiles * SYM_T;
+    b.ts.pack.ensure<float4>(padded);
+    b.ts.eps.ensure<float>(padded);
+    b.ts.meta.ensure<float4>(2 * (size_t)b.ntiles);
+    b.ts.idx.ensure<uint32_t>(padded);
+    b.ts.resid.ensure<float4>(padded);
+    b.ts.sub.ensure<float4>(2 * (padded / SUBTILE));
+    b.part.ensure<double>(part);
+    b.ens_ctl.ensure<unsigned>(1 + 2 * (size_t)b.count + b.ntiles);
+    STEPS_CUDA(cudaMemcpyAsync(b.tdesc.ensure<int2>(desc.size()), desc.data(), desc.size() * sizeof(int2),
+                               cudaMemcpyHostToDevice, c.stream));
+    STEPS_CUDA(cudaMemcpyAsync(b.rels.ensure<EnsRel>(rel.size()), rel.data(), rel.size() * sizeof(EnsRel),
+                               cudaMemcpyHostToDevice, c.stream));
+    STEPS_CUDA(cudaMemcpyAsync(b.tasks.ensure<int4>(tasks.size()), tasks.data(), tasks.size() * sizeof(int4),
+                               cudaMemcpyHostToDevice, c.stream));
+    STEPS_CUDA(cudaStreamSynchronize(c.stream));
 }
 
-// Times one force evaluation (a one-stage run) per candidate tile shape,
-// j-chunk length and grid size, and keeps the fastest.
+// The same with the slabs within 16 GiB, or less where that does not fit.
+void ensemble_plan(Batch &b, int NP, int split)
+{
+    int most = (int)std::min(128.0, std::max(4.0, (double)(16LL << 30) / (24.0 * b.ntot) / 1.5));
+    for (;;) {
+        try {
+            ensemble_plan_most(b, NP, split, most);
+            return;
+        } catch (const Error &e) {
+            if (e.code != STEPS_E_NOMEM || most <= 1) throw;
+            most /= 2;
+        }
+    }
+}
+
+// Times three stages (two steps of length 0, which leave positions and velocities
+// as they are) per row width and item size, and keeps the fastest: one stage
+// alone overrates small items, which end evenly but cost more slabs.
 void ensemble_tune(Batch &b)
 {
     Ctx &c = ctx();
-    static const int shapes[][2] = {{128, 2}, {128, 1}, {256, 1}, {64, 2}};
-    static const int jmaxes[] = {64, 256};
-    static const double fracs[] = {1.0, 0.75};
+    static const int splits[] = {6, 16, 40};
     float best = 1e30f;
-    int bt = 128, bi = 2, bj = 256;
-    double bf = 1.0;
-    for (auto &sh : shapes)
-        for (int jm : jmaxes)
-            for (double fr : fracs) {
-                ensemble_plan(b, sh[0], sh[1], jm, fr);
-                ensemble_run(b, 0, 0.0, -1);  // warm
-                STEPS_CUDA(cudaEventRecord(c.marks[12], c.stream));
-                ensemble_run(b, 0, 0.0, -1);
-                STEPS_CUDA(cudaEventRecord(c.marks[13], c.stream));
-                STEPS_CUDA(cudaEventSynchronize(c.marks[13]));
-                float ms = 0;
-                STEPS_CUDA(cudaEventElapsedTime(&ms, c.marks[12], c.marks[13]));
-                if (ms < best) { best = ms; bt = sh[0]; bi = sh[1]; bj = jm; bf = fr; }
-            }
+    int bn = 2, bs = 16;
+    for (int np = 2; np <= 4; np += 2)
+        for (int sp : splits) {
+            ensemble_plan(b, np, sp);
+            ensemble_run(b, 0, 0.0, -1);  // warm
+            STEPS_CUDA(cudaEventRecord(c.marks[12], c.stream));
+            ensemble_run(b, 2, 0.0, -1);
+            STEPS_CUDA(cudaEventRecord(c.marks[13], c.stream));
+            STEPS_CUDA(cudaEventSynchronize(c.marks[13]));
+            float ms = 0;
+            STEPS_CUDA(cudaEventElapsedTime(&ms, c.marks[12], c.marks[13]));
+            if (ms < best) { best = ms; bn = np; bs = sp; }
+        }
     check_kernel_status();
-    ensemble_plan(b, bt, bi, bj, bf);
-    b.ens_threads = bt;
-    b.ens_ipt = bi;
-    b.ens_jmax = bj;
-    b.ens_frac = bf;
+    ensemble_plan(b, bn, bs);
     b.ens_tuned = true;
 }
 
@@ -444,8 +473,7 @@ void batch_release()
     DevBuf *bufs[] = {&b->x, &b->v, &b->F, &b->m64, &b->eps64, &b->rel, &b->bbox, &b->tdesc, &b->items, &b->tslot,
                       &b->part, &b->counter, &b->err, &b->ts.keys[0], &b->ts.keys[1], &b->ts.vals[0], &b->ts.vals[1],
                       &b->ts.hist, &b->ts.pack, &b->ts.eps, &b->ts.meta, &b->ts.idx, &b->ts.resid, &b->ts.soa,
-                      &b->ts.sub, &b->pack2, &b->soa2, &b->resid2, &b->meta2, &b->sub2, &b->tile_rel,
-                      &b->rel_ntiles, &b->ens_ctl};
+                      &b->ts.sub, &b->rels, &b->tasks, &b->ens_ctl};
     for (DevBuf *d : bufs) d->release();
     delete b;
     c.batch = nullptr;
@@ -561,7 +589,7 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
                 const int k = b.stall_rel;
                 b.stall_rel = -1;
                 if (!b.ens_tuned) ensemble_tune(b);
-                else ensemble_plan(b, b.ens_threads, b.ens_ipt, b.ens_jmax, b.ens_frac);
+                else ensemble_plan(b, b.ens_np, b.ens_split);
                 release_graph(b);
                 ensemble_run(b, a.nsteps, a.h, k);
                 STEPS_CUDA(cudaStreamSynchronize(c.stream));
@@ -597,7 +625,7 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
             if (!b.exec || b.graph_steps != a.nsteps || b.graph_h != a.h || b.graph_mode != a.graph) {
                 release_graph(b);
                 // the plan of the chosen path (the two paths keep their own shapes)
-                if (persistent) ensemble_plan(b, b.ens_threads, b.ens_ipt, b.ens_jmax, b.ens_frac);
+                if (persistent) ensemble_plan(b, b.ens_np, b.ens_split);
                 else plan(b, b.threads_pp, b.ipt_pp);
                 if (!persistent) batch_forces(b);  // sizes every buffer before capture
                 kernel_status_word();              // allocated outside the capture

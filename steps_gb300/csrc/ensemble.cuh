@@ -1,0 +1,44 @@
+// The persistent ensemble kernel (ensemble.cu): every force evaluation and KDK
+// step of a batch of R^3 realisations in one launch.
+#pragma once
+
+#include "common.cuh"
+#include "sym.cuh"
+
+namespace steps {
+
+// One realisation: its tiles (padded to whole rows), the split of its pairs
+// (SymPlan) and its slabs of partial sums.
+struct EnsRel {
+    int tile0, ntiles;            // first tile of the batch arrays; tiles that hold particles
+    int nrows, G, C, step, gran;  // as in SymArgs / SymPlan
+    int npair;                    // pair tasks of a stage; finish tasks: 4 ntiles
+    size_t npad;
+    size_t part;                  // first double of its slabs
+};
+
+struct EnsembleArgs {
+    const EnsRel *rel;
+    const int4 *tasks;      // of one stage: (realisation, group, chunk, 0) or (realisation, 32 particles, 0, 1)
+    int ntasks, nstages, nrel;
+    float4 *pack, *resid, *meta, *sub;
+    const float *eps;       // softening (constant over the run)
+    const uint32_t *idx;    // original index of each padded position (constant)
+    double *part;
+    unsigned *queue;        // task counter
+    unsigned *pair_done, *fin_done;  // per realisation: items, tiles done, over all stages
+    unsigned *tile_cnt;     // per tile: finish tasks done, over all stages
+    double *x, *v, *F;      // caller-order FP64 positions, velocities, forces
+    double h;               // fixed step; acceleration g F a^-3 - 2 H v with g = 1, a = 1, H = 0
+    float guard2;
+    int n, ntiles;
+    long long wait_cycles;  // SM clock cycles after which a wait gives up
+    int *status;            // STEPS_E_TIMEOUT when a wait gave up
+    int stall_rel;          // test hook: this realisation's stage-0 tiles are never reported done (-1: none)
+};
+
+// Launches the kernel with rows of 64 NP particles (NP 2 or 4).
+void ensemble_launch(int NP, const EnsembleArgs &e, cudaStream_t st);
+int ensemble_blocks(int NP);  // resident blocks per SM
+
+}  // namespace steps

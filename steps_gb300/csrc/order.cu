@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(TB_THREADS) k_tile_build(const double *__restr
 #ifdef STEPS_CHECK
     if (!check_span(sbase, (long long)sbase + cnt - 1, count, CK_PERM)) cnt = 0;
 #endif
-    build_tile<TB_THREADS, false>(tile, sbase, cnt, x, m, eps, perm, nx, T, pack, epsf, meta, idx, pad_id, lo, soa,
+    build_tile<TB_THREADS>(tile, sbase, cnt, x, m, eps, perm, nx, T, pack, epsf, meta, idx, pad_id, lo, soa,
                                   sub);
 }
 

@@ -1,6 +1,6 @@
-// The tile builder shared by the ordering pass (order.cu) and the persistent
-// ensemble kernel (pair_r3x2.cu), which rebuilds each tile after its kick and
-// drift.
+// The tile builder of the ordering pass (order.cu). The persistent ensemble
+// kernel (ensemble.cu) rebuilds its tiles with the same arithmetic, one warp to
+// a tile.
 #pragma once
 
 #include "common.cuh"
@@ -23,9 +23,7 @@ __device__ __forceinline__ double warp_max(double v)
 // largest softening (meta), FP32 offsets (pack, soa), their FP32 residuals
 // (lo), softening (epsf), original indices (idx) and the sub-tile boxes (sub).
 // perm holds original indices below nx (checked in bounds-checked builds).
-// COH: positions are read through L2 (ld.global.cg), for a kernel in which
-// other blocks have just written them (L1 is not coherent across SMs).
-template <int NT, bool COH>
+template <int NT>
 __device__ __forceinline__ void build_tile(int tile, int sbase, int cnt, const double *__restrict__ x,
                                            const double *__restrict__ m, const double *__restrict__ eps,
                                            const uint32_t *__restrict__ perm, long long nx, int T,
@@ -36,7 +34,6 @@ __device__ __forceinline__ void build_tile(int tile, int sbase, int cnt, const d
 {
     __shared__ double red[7][NT / 32];
     __shared__ float s_c[3];
-    auto ldx = [&](size_t q) { return COH ? __ldcg(x + q) : x[q]; };
     int t = threadIdx.x, lane = t & 31, w = t >> 5;
     double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, em = 0.0;
     for (int e = t; e < T; e += NT) {
@@ -44,7 +41,7 @@ __device__ __forceinline__ void build_tile(int tile, int sbase, int cnt, const d
             uint32_t o = perm[sbase + e];
             STEPS_CHECK_IDX(o, nx, CK_PERM);
             for (int k = 0; k < 3; k++) {
-                double v = ldx(3 * (size_t)o + k);
+                double v = x[3 * (size_t)o + k];
                 mn[k] = fmin(mn[k], v);
                 mx[k] = fmax(mx[k], v);
             }
@@ -84,7 +81,7 @@ __device__ __forceinline__ void build_tile(int tile, int sbase, int cnt, const d
         if (e < cnt) {
             uint32_t o = perm[sbase + e];
             STEPS_CHECK_IDX(o, nx, CK_PERM);
-            const double ox = ldx(3 * (size_t)o) - cx, oy = ldx(3 * (size_t)o + 1) - cy, oz = ldx(3 * (size_t)o + 2) - cz;
+            const double ox = x[3 * (size_t)o] - cx, oy = x[3 * (size_t)o + 1] - cy, oz = x[3 * (size_t)o + 2] - cz;
             const float hx = __double2float_rn(ox), hy = __double2float_rn(oy), hz = __double2float_rn(oz);
             pack[q] = make_float4(hx, hy, hz, __double2float_rn(m[o]));
             if (soa) {  // tile-blocked SoA copy: X[T], Y[T], Z[T], M[T] per tile
