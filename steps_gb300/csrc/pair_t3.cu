@@ -218,88 +218,8 @@ __global__ void __launch_bounds__(BLOCK) k_pair_t3(MixedArgs a)
                             const float4 *base = win + (bx * sx + by * sy + bz);
                             stencil<ORDER>(wx, wy, wz, [&](int aa, int bb, int cc) { return base[aa * sx + bb * sy + cc]; },
                                            Dx, Dy, Dz);
-                        } else if (halo) {  // haloed table in L1/L2, no wrap
-                            const float uh = a.u0 + (float)a.halo;
-                            const float ux = fmaf(dx, a.ih, uh), uy = fmaf(dy, a.ih, uh), uz = fmaf(dz, a.ih, uh);
-                            const float fxl = floorf(ux), fyl = floorf(uy), fzl = floorf(uz);
-                            weights<ORDER>(ux - fxl, wx);
-                            weights<ORDER>(uy - fyl, wy);
-                            weights<ORDER>(uz - fzl, wz);
-                            const int E = a.ext;
-                            bx = min(max((int)fxl - OFF, 0), E - NT);
-                            by = min(max((int)fyl - OFF, 0), E - NT);
-                            bz = min(max((int)fzl - OFF, 0), E - NT);
-#ifdef STEPS_CHECK
-                            const long long hfirst = ((long long)bx * E + by) * E + bz;
-                            if (!check_span(hfirst, hfirst + (long long)(NT - 1) * ((long long)E * E + E + 1),
-                                            (long long)E * E * E, CK_T3_CELL))
-                                bx = by = bz = 0;
-#endif
-                            if (ORDER == 4) {
-                                // z-row records: the 4 z taps of one (x, y) row, per
-                                // component, in 3 float4 (48 B), 16 rows per pair
-                                const int cb = (bx * E + by) * E + bz;
-#pragma unroll
-                                for (int aa = 0; aa < 4; aa++) {
-                                    float rx = 0.0f, ry = 0.0f, rz = 0.0f;
-#pragma unroll
-                                    for (int bb = 0; bb < 4; bb++) {
-                                        const int cr = cb + (aa * E + bb) * E;
-                                        float4 vx, vy;
-                                        ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
-                                        const float4 vz = __ldg(a.t3rz + cr);
-                                        rx = fmaf(wy[bb], dot4(wz, vx), rx);
-                                        ry = fmaf(wy[bb], dot4(wz, vy), ry);
-                                        rz = fmaf(wy[bb], dot4(wz, vz), rz);
-                                    }
-                                    Dx = fmaf(wx[aa], rx, Dx);
-                                    Dy = fmaf(wx[aa], ry, Dy);
-                                    Dz = fmaf(wx[aa], rz, Dz);
-                                }
-                            } else {
-                                // (y, z) quad records: cells (x, y..y+1, z..z+1), per
-                                // component, in 3 float4 (48 B), 2 records per pair
-                                const float q00 = wy[0] * wz[0], q01 = wy[0] * wz[1], q10 = wy[1] * wz[0],
-                                            q11 = wy[1] * wz[1];
-                                const int cb = (bx * E + by) * E + bz;
-#pragma unroll
-                                for (int aa = 0; aa < 2; aa++) {
-                                    const int cr = cb + aa * E * E;
-                                    float4 vx, vy;
-                                    ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
-                                    const float4 vz = __ldg(a.t3rz + cr);
-                                    Dx = fmaf(wx[aa], fmaf(q11, vx.w, fmaf(q10, vx.z, fmaf(q01, vx.y, q00 * vx.x))), Dx);
-                                    Dy = fmaf(wx[aa], fmaf(q11, vy.w, fmaf(q10, vy.z, fmaf(q01, vy.y, q00 * vy.x))), Dy);
-                                    Dz = fmaf(wx[aa], fmaf(q11, vz.w, fmaf(q10, vz.z, fmaf(q01, vz.y, q00 * vz.x))), Dz);
-                                }
-                            }
-                        } else {  // wrapped lookup (tile pairs wider than the halo)
-                            const float ux = fmaf(dx, a.ih, a.u0), uy = fmaf(dy, a.ih, a.u0),
-                                        uz = fmaf(dz, a.ih, a.u0);
-                            const float fxl = floorf(ux), fyl = floorf(uy), fzl = floorf(uz);
-                            weights<ORDER>(ux - fxl, wx);
-                            weights<ORDER>(uy - fyl, wy);
-                            weights<ORDER>(uz - fzl, wz);
-                            bx = (int)fxl - OFF;
-                            by = (int)fyl - OFF;
-                            bz = (int)fzl - OFF;
-                            // Stencil indices wrapped once per axis: |d| < 3L/2,
-                            // so every index lies in [-2 ng, 3 ng).
-                            int gx[NT], gy[NT], gz[NT];
-#pragma unroll
-                            for (int t = 0; t < NT; t++) {
-                                gx[t] = wrap_index(bx + t, a.ng) + a.halo;
-                                gy[t] = wrap_index(by + t, a.ng) + a.halo;
-                                gz[t] = wrap_index(bz + t, a.ng) + a.halo;
-                                STEPS_CHECK_IDX(gx[t], a.ext, CK_T3_CELL);
-                                STEPS_CHECK_IDX(gy[t], a.ext, CK_T3_CELL);
-                                STEPS_CHECK_IDX(gz[t], a.ext, CK_T3_CELL);
-                            }
-                            stencil<ORDER>(wx, wy, wz,
-                                           [&](int aa, int bb, int cc) {
-                                               return __ldg(a.t3f + (gx[aa] * a.ext + gy[bb]) * a.ext + gz[cc]);
-                                           },
-                                           Dx, Dy, Dz);
+                        } else if constexpr (ORDER != 0) {  // haloed table in L1/L2
+                            t3_correction<ORDER>(a, halo, dx, dy, dz, Dx, Dy, Dz);
                         }
                     }
                     fx[k] = fmaf(q.w, fmaf(w, nx, -Dx), fx[k]);
@@ -812,26 +732,28 @@ KernelFn t3_kernel(const KParams &kp, int threads, int ipt, size_t *dyn_smem, in
     return kp.order == 4 ? pick_t3<4>(threads, ipt) : pick_t3<2>(threads, ipt);
 }
 
-// Stencil records of the haloed table, one float4 per component, record
-// (i, j, k) of the ext^3 grid (x and y in out[2c], out[2c + 1], z in outz[c]):
+// Stencil records of the haloed table, one float4 per component, for the cell
+// (i, j, k) of the ext^3 grid at index t3_record(i, j, k) (x and y in out[2c],
+// out[2c + 1], z in outz[c]):
 //   tricubic: z row  -- cells (i, j, k..k+3)
 //   trilinear: (y, z) quad -- cells (i, j, k), (i, j, k+1), (i, j+1, k), (i, j+1, k+1)
+// One thread per cell; the last brick's cells beyond an odd ext are never read.
 __global__ void k_table_records(const double *__restrict__ t, int ng, int halo, int order, float4 *__restrict__ out,
                                 float4 *__restrict__ outz)
 {
     const int ext = ng + 2 * halo;
-    const size_t ncell = (size_t)ext * ext * ext;
-    size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int k = (int)(c % ext), j = (int)((c / ext) % ext), i = (int)(c / ((size_t)ext * ext));
+    const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= (size_t)ext * ext * ext) return;
+    const int k = (int)(n % ext), j = (int)((n / ext) % ext), i = (int)(n / ((size_t)ext * ext));
+    const int c = order == 4 ? t3_record<4>(i, j, k, ext) : t3_record<2>(i, j, k, ext);
     float v[3][4];
     for (int q = 0; q < 4; q++) {
         const int dj = order == 4 ? 0 : q >> 1, dk = order == 4 ? q : q & 1;
         const size_t s = ((size_t)pmod(i - halo, ng) * ng + pmod(j + dj - halo, ng)) * ng + pmod(k + dk - halo, ng);
         for (int comp = 0; comp < 3; comp++) v[comp][q] = (float)t[3 * s + comp];
     }
-    out[2 * c] = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-    out[2 * c + 1] = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+    out[2 * (size_t)c] = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+    out[2 * (size_t)c + 1] = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
     outz[c] = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
 }
 
@@ -839,6 +761,12 @@ __global__ void k_table_records(const double *__restrict__ t, int ng, int halo, 
 // need no per-pair wrap. It grows with the grid (cells shrink as L / ng, tile
 // extents do not): 16 cells at ng = 63, ng / 8 above 128.
 inline int t3_halo(int ng) { return ng / 8 > 16 ? ng / 8 : 16; }
+// Room for the stencil records: an even extent holds whole bricks.
+inline size_t t3_records(int ng)
+{
+    const size_t e = ((size_t)ng + 2 * t3_halo(ng) + 1) / 2 * 2;
+    return e * e * e;
+}
 
 // FP32 float4 haloed copy of the FP64 table, rebuilt whenever the table changes.
 const float4 *t3_table_f32(const Tables &tb, cudaStream_t st)
@@ -860,12 +788,12 @@ const float4 *t3_table_f32(const Tables &tb, cudaStream_t st)
 const float4 *t3_table_records(const Tables &tb, int order, cudaStream_t st)
 {
     Ctx &c = ctx();
-    const size_t ext = (size_t)tb.t3_ng + 2 * t3_halo(tb.t3_ng);
-    const size_t ncell = ext * ext * ext;
+    const size_t nrec = t3_records(tb.t3_ng);
     if (c.t3r_version != c.t3_version || c.t3r_order != order || !c.t3r.p) {
-        float4 *o = c.t3r.ensure<float4>(3 * ncell);  // 2 ncell xy records, then ncell z records
+        float4 *o = c.t3r.ensure<float4>(3 * nrec);  // 2 nrec xy records, then nrec z records
+        const size_t ext = (size_t)tb.t3_ng + 2 * t3_halo(tb.t3_ng), ncell = ext * ext * ext;
         k_table_records<<<(unsigned)((ncell + 255) / 256), 256, 0, st>>>(tb.t3, tb.t3_ng, t3_halo(tb.t3_ng), order,
-                                                                          o, o + 2 * ncell);
+                                                                          o, o + 2 * nrec);
         note_launch("k_table_records");
         c.t3r_version = c.t3_version;
         c.t3r_order = order;
@@ -887,8 +815,7 @@ void t3_args(MixedArgs &a, const KParams &kp, const Tables &tb, cudaStream_t st)
     if (kp.is_periodic >= 2) {
         a.t3f = t3_table_f32(tb, st);
         a.t3r = t3_table_records(tb, kp.order == 4 ? 4 : 2, st);
-        const size_t ext = (size_t)tb.t3_ng + 2 * t3_halo(tb.t3_ng);
-        a.t3rz = a.t3r + 2 * ext * ext * ext;
+        a.t3rz = a.t3r + 2 * t3_records(tb.t3_ng);
         a.ih = (float)((double)tb.t3_ng / kp.L);
         a.u0 = (float)((double)tb.t3_ng * 0.5 - 0.5);
     }

@@ -42,11 +42,27 @@ __device__ __forceinline__ void weights(float t, float *w)
 }
 
 // T^3 stencil records, one float4 per component, in two arrays of the same
-// cell index: the x and y components as one 32-byte record (a.t3r, read with
+// record index: the x and y components as one 32-byte record (a.t3r, read with
 // one 256-bit load) and the z component as one 16-byte record (a.t3rz): two
 // L1 requests per record instead of three, in the same 48 bytes per cell.
 // (Records padded to 64 bytes for the same purpose were 13-17 % slower: the
 // larger table loses L1 hits.)
+//
+// Index of the record of cell (x, y, z) of the haloed table of extent E. The L1
+// path, which bounds the table kernels, takes one cycle per 128-byte line that a
+// group of 4 (256-bit) or 8 (128-bit) lanes touches, and the lanes' cells spread
+// over all three axes. Trilinear: bricks of 2 x 2 x 2 cells (40,961 particles,
+// pairwise kernel, against rows along z: 6.59 / 6.93 ms at ng = 63, 10.97 / 11.80
+// ms at ng = 127; one-sided 17.34 / 17.58 and 23.96 / 24.46). Tricubic: rows along
+// z, since its 16 records need 8 indices instead of one (pairwise 52.8 ms, bricks
+// 52.1; one-sided 124.4 ms, bricks 138.4).
+template <int ORDER>
+__host__ __device__ __forceinline__ int t3_record(int x, int y, int z, int E)
+{
+    if (ORDER == 4) return (x * E + y) * E + z;
+    const int H = (E + 1) >> 1;
+    return ((((x >> 1) * H + (y >> 1)) * H + (z >> 1)) << 3) + ((x & 1) << 2) + ((y & 1) << 1) + (z & 1);
+}
 
 // Two float4 of a 32-byte aligned record in one 256-bit load (sm_100+):
 // the L1 data path, which bounds the table kernels, sees one request per
@@ -223,14 +239,13 @@ __device__ __forceinline__ void t3_correction(const MixedArgs &a, bool halo, flo
                         CK_T3_CELL))
             bx = by = bz = 0;
 #endif
-        const int cb = (bx * E + by) * E + bz;
         if (ORDER == 4) {  // z-row records
 #pragma unroll
             for (int aa = 0; aa < 4; aa++) {
                 float rx = 0.0f, ry = 0.0f, rz = 0.0f;
 #pragma unroll
                 for (int bb = 0; bb < 4; bb++) {
-                    const int cr = cb + (aa * E + bb) * E;
+                    const int cr = t3_record<4>(bx + aa, by + bb, bz, E);
                     float4 vx, vy;
                     ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
                     const float4 vz = __ldg(a.t3rz + cr);
@@ -246,7 +261,7 @@ __device__ __forceinline__ void t3_correction(const MixedArgs &a, bool halo, flo
             const float q00 = wy[0] * wz[0], q01 = wy[0] * wz[1], q10 = wy[1] * wz[0], q11 = wy[1] * wz[1];
 #pragma unroll
             for (int aa = 0; aa < 2; aa++) {
-                const int cr = cb + aa * E * E;
+                const int cr = t3_record<2>(bx + aa, by, bz, E);
                 float4 vx, vy;
                 ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
                 const float4 vz = __ldg(a.t3rz + cr);

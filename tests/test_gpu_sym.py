@@ -127,6 +127,19 @@ def test_periodic_sizes(fresh, kind, n):
     assert np.array_equal(F, fresh.forces(ps.x, p, S.MIXED))
 
 
+@pytest.mark.parametrize("ng", [5, 31, 129, 145])
+@pytest.mark.parametrize("n", [1500, 4500])
+def test_t3_brick_records(fresh, ng, n):
+    """Trilinear records in bricks: grids of 1 and 3 (mod 4) cells, halo of 16 cells and wider; one-sided and
+    pairwise, and particles over the whole box, so that cells at the edges of the haloed table are read."""
+    ps = W.t3_clumpy(n, L3, 5)
+    fresh.build_table_t3(ng, L3, 2.0 / L3, 2.0, 5.0 * 2.0 * math.pi / L3, 3.0, 6.0)
+    p = S.params(S.T3, is_periodic=2, L=L3, rsim=L3 / 2, ewald_order=2)
+    fresh.set_particles(ps.m, ps.eps)
+    st = err_stats(fresh.forces(ps.x, p, S.MIXED), fresh.forces(ps.x, p, S.FP64))
+    assert st["p99"] < MIXED_P99, (ng, n, st)
+
+
 @pytest.mark.parametrize("kind", KINDS)
 def test_periodic_hard_decisions(fresh, kind):
     """Pairs within a few FP32 ulps of half a period along each axis and of the image cut: the image is the FP64
