@@ -111,7 +111,7 @@ constexpr int SYM_MIN_N = 16384;
 constexpr int SYM_FP64_MIN_N = 512;
 constexpr int BOX_MIN_N = 4096;  // periodic topologies (n = 3,000 / 5,000, one-sided tuned -> pairwise, us: trilinear 189 /
                                // 393 -> 175 / 251, CIC 66 / 143 -> 101 / 119, images 95 / 179 -> 99 / 132)
-constexpr int SYM_NP4_N = 40000;  // from here on rows of 256 particles instead of 128
+constexpr int SYM_NP4_N = 100000;  // from here on rows of 256 particles instead of 128
 constexpr long long SYM_PARTIAL_BYTES = 16LL << 30;  // FP64 partial sums of both sides at most
 bool sym_supported(const KParams &kp, const Tables &tb, int n);
 // A mixed call: the pairwise kernel where the call and the shape allow it, else (or where its partial sums do not fit

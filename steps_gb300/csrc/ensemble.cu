@@ -184,7 +184,7 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
 }
 
 template <int NP>
-__global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_ensemble(EnsembleArgs e)
+__global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(EnsembleArgs e)
 {
     __shared__ __align__(16) SymWarp<NP> shw[SYM_WARPS];
     __shared__ SymArgs sha[SYM_WARPS];  // each warp's item, out of the pair loop's registers

@@ -37,11 +37,15 @@
 // of the one-sided kernels and take the double-float path, after the far ones.
 //
 // Measured (GB300, clustered compactified sets, pair kernel, one-sided packed
-// kernel -> this one): n = 32,768: 628 (tuned 525) -> 421 us; 262,144:
-// 28.3 -> 19.4 ms; 2^20: 404 -> 297 ms, the FMA pipe 77 % busy.
-// Further warps per SM (fewer registers, NP = 2), scalar instead of packed
-// sums, other unrollings and a single rotated sum instead of two all measured
-// within 3 % or slower: the FMA pipe with its operand reads is the limit.
+// kernel -> this one): n = 32,768: 628 (tuned 525) -> 416 us; 262,144:
+// 28.3 -> 19.0 ms; 2^20: 404 -> 293 ms, the FMA pipe 77 % busy.
+// Scalar instead of packed sums and a single rotated sum instead of two
+// measured within 3 % or slower: the FMA pipe with its operand reads is the
+// limit. 16 warps an SM with all the registers they want do better than more:
+// NP = 2, 6 blocks of 80 registers 433 us at n = 32,768 and 648 at 39,999, 5
+// blocks 422 and 624, 4 blocks 416 and 613 (3: 449 and 650). The rotation is
+// unrolled 16 times (8 / 16 / 32 times: NP = 2, n = 32,768 420 / 416 / 449 us;
+// NP = 4, n = 262,144 19.37 / 19.02 / 25.1 ms).
 #include <algorithm>
 
 #include "common.cuh"
@@ -58,7 +62,7 @@ namespace {
 using namespace mixed;
 
 template <int NP>
-__global__ void __launch_bounds__(SYM_THREADS, NP == 4 ? 4 : 6) k_sym_r3(SymArgs a)
+__global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_sym_r3(SymArgs a)
 {
     __shared__ __align__(16) SymWarp<NP> shw[SYM_WARPS];
     const int lane = threadIdx.x & 31;
@@ -134,9 +138,10 @@ bool sym_split(SymPlan &p, int tile)
 
 namespace {
 
-// Row width for n particles. Narrow rows give small sets enough warps, wide ones
-// amortise the rotation (pair kernel, NP = 2 / 4: n = 32,768 427 / 458 us;
-// 48,000 853 / 818; 131,072 5434 / 5111).
+// Row width for n particles. Narrow rows give small sets enough items, wide ones
+// amortise the rotation (pair kernel and reduction, NP = 2 / 4: n = 48,000
+// 0.894 / 0.911 ms; 72,000 1.821 / 1.883; 90,000 2.710 / 2.727; 110,000
+// 3.897 / 3.867; 131,072 5.41 / 5.29).
 bool sym_plan(int n, SymPlan &p)
 {
     p.NP = n >= SYM_NP4_N ? 4 : 2;

@@ -10,6 +10,7 @@ namespace steps {
 constexpr int SYM_T = 128;                 // particles per tile
 constexpr int SYM_WARPS = 4;               // per block; each works on its own
 constexpr int SYM_THREADS = 32 * SYM_WARPS;
+constexpr int SYM_R3_BLOCKS = 4;  // per SM asked of the register allocator: 128 registers a thread
 constexpr int SYM_HALF = SYM_T / 2;
 constexpr int SYM_NSUB = SYM_T / SUBTILE;  // 8 sub-tile boxes per tile
 

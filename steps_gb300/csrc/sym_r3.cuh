@@ -79,11 +79,12 @@ __device__ __forceinline__ void frame_offset(const SymArgs &a, int J, int H, flo
     dO[2] = two_diff(mJ.z, mI.z, eO[2]);
 }
 
-// The group of 32 j particles in shared memory (lane l's own is entry l) against the slots 2h,
-// 2h + 1 of this warp, pair by pair in double-float coordinates with the
-// softening spline: the exact path of r3x2_tile, rotated like the far loop.
-// Lane l starts at entry l and moves on by one entry a step. near = false runs the far arithmetic instead (a far slot pair of a group
-// that has near ones). The i sums go to the FP64 accumulators, the j sums to
+// The group of 32 j particles in shared memory (lane l's own is entry l)
+// against the slots 2h, 2h + 1 of this warp, pair by pair in double-float
+// coordinates with the softening spline: the exact path of r3x2_tile, rotated
+// like the far loop. Lane l starts at entry l and moves on by one entry a step.
+// near = false runs the far arithmetic instead (a far slot pair of a group that
+// has near ones). The i sums go to the FP64 accumulators, the j sums to
 // (jx, jy, jz).
 template <int NP, bool COH>
 __device__ __forceinline__ void r3_slots(const SymArgs &a, SymWarp<NP> &sh, int H, int h, bool near,
@@ -259,7 +260,7 @@ __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int 
                 sh.q[lane] = sh.q[32 + lane] = q0;
                 __syncwarp();
                 f2 JX = 0ull, JY = 0ull, JZ = 0ull;
-#pragma unroll 8
+#pragma unroll 16
                 for (int s = 0; s < 32; s++) {
                     const float4 q = sh.q[lane + s];
                     const f2 qx = f2_bcast(q.x), qy = f2_bcast(q.y), qz = f2_bcast(q.z), qm = f2_bcast(q.w);

@@ -24,7 +24,7 @@ def fresh(engine):
     eng.set_variant(0)
 
 
-@pytest.mark.parametrize("n", [16384, 16385, 16511, 20001, 39999, 40000, 65600, 70001])
+@pytest.mark.parametrize("n", [16384, 16385, 16511, 20001, 39999, 40000, 65600, 70001, 99999, 100000, 100353])
 def test_r3_sizes(fresh, n):
     """Taken from n = 16,384 on; wider rows from 40,000 on, groups of several rows from 32,769 (narrow) and 65,537 on."""
     ps = W.r3_compactified(n, 480.0, seed=n, displace=True)
