@@ -245,7 +245,7 @@ int steps_gpu_batch_get(int k, double *x, double *v, double *F);
  * is threads*ipt. Returns STEPS_E_ARG for an unsupported shape. A shape or
  * variant (steps_gpu_set_kernel_variant) set explicitly is used as given;
  * without one, and after steps_gpu_autotune, calls for the forces of all
- * particles (from 16,384 on in R^3, 4,096 on in the periodic topologies) run a
+ * particles (from 20,000 on in R^3, 4,096 on in the periodic topologies) run a
  * kernel that evaluates each pair once for both particles; with a correction
  * table only if the table is odd in the separation, as the builders' are. */
 int steps_gpu_set_tuning(int threads, int ipt, int jsplit);

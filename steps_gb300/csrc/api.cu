@@ -589,8 +589,8 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
         KParams kp = derive_params(p);
         if (sym_call(kp, device_tables(kp), c.n, id_min, id_max - id_min + 1)) {
             // The pairwise kernels are at least as fast as every one-sided
-            // shape at the sizes they take (R^3: within 3 % at n = 16,384, 1.2
-            // times from 32,768 on, 1.35 times at 2^20; periodic: 1.1-1.8 times
+            // shape at the sizes they take (R^3: equal at n = 20,000, 1.25
+            // times at 32,768, 1.38 times at 2^20; periodic: 1.1-1.8 times
             // at 5,000, about twice from 8,000 on), so nothing is timed; one
             // evaluation sizes the buffers.
             const bool keep_sym = c.shape.sym;

@@ -104,10 +104,10 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
                   int n, int id_min, int ni, double *F, bool reuse_order);
 // pair_sym.cu: full-range mixed forces with every pair of particles evaluated
 // once. sym_supported: the calls it takes.
-// From SYM_MIN_N on: below, the one-sided kernels with small tiles fill the GPU
-// better (n = 8,192: 70 us against 99; 12,000: 124 against 127; 16,384: 181
-// against 186, tuned; 24,000: 328 against 312, pair kernel and reduction).
-constexpr int SYM_MIN_N = 16384;
+// From SYM_MIN_N on: below, the one-sided kernels with small tiles and few
+// partial sums are better (whole evaluation, us: n = 16,384 215 against 233;
+// 20,000 300 against 303; 24,000 377 against 365; 28,000 480 against 441).
+constexpr int SYM_MIN_N = 20000;
 constexpr int SYM_FP64_MIN_N = 512;
 constexpr int BOX_MIN_N = 4096;  // periodic topologies (n = 3,000 / 5,000, one-sided tuned -> pairwise, us: trilinear 189 /
                                // 393 -> 175 / 251, CIC 66 / 143 -> 101 / 119, images 95 / 179 -> 99 / 132)

@@ -502,10 +502,12 @@ void period_args(mixed::MixedArgs &a, const KParams &kp)
 bool mixed_supported(const KParams &kp) { return select_kernel(kp, 128, 2) != nullptr; }
 
 // The one-sided kernel shape where the caller chose none, for ni particles
-// against n. R^3: small tiles give small calls enough items; from 2.5e7 pairs
-// on 256 x 1 at 1024 threads an SM, from 8e9 on 128 x 2 (measured, us, 128 x 2
-// scalar -> this: 2,000^2 160 -> 15, 3,001^2 151 -> 24, 3,000 x 30,000 189 ->
-// 89, 20,000 x 100,000 1424 -> 962, 66,667 x 200,003 7401 -> 5600). Periodic:
+// against n. R^3: small tiles give small calls enough items, at 1024 threads an
+// SM: 64 x 1 below 3e7 pairs, 128 x 1 below 1.5e8, 256 x 1 below 8e9, then
+// 128 x 2 at 640 (pair kernel and reduction, us, 64 x 1 / 128 x 1 / 256 x 1:
+// 3,001^2 29 / 31 / 42; 5,000^2 44 / 48 / 48; 8,000^2 72 / 66 / 87; 12,000^2 130
+// / 113 / 117; 2,000 x 100,000 216 / 175 / 171; 20,000 x 200,000 2157 / 1964 /
+// 1892; 66,667 x 200,003 7401 with 128 x 2 scalar, 5600 packed). Periodic:
 // 64 x 1, whose smaller boxes send fewer pairs down the near path (33,333 x
 // 100,000, ms, 128 x 2 -> 64 x 1: trilinear 34.0 -> 29.3, images 17.8 -> 8.8,
 // nearest image 6.1 -> 3.7); from 1e9 pairs on 256 x 1 for the wide stencils,
@@ -515,9 +517,9 @@ Shape auto_shape(const KParams &kp, int ni, int n)
     Shape s = ctx().shape;
     const double pairs = (double)ni * (double)n;
     if (kp.topology == STEPS_R3) {
-        s.threads = pairs < 2.5e7 ? 64 : pairs < 8e9 ? 256 : 128;
+        s.threads = pairs < 3e7 ? 64 : pairs < 1.5e8 ? 128 : pairs < 8e9 ? 256 : 128;
         s.ipt = pairs < 8e9 ? 1 : 2;
-        s.variant = pairs < 2.5e7 || pairs >= 8e9 ? 1 : 3;
+        s.variant = pairs < 8e9 ? 3 : 1;
         return s;
     }
     if (kp.topology == STEPS_T3 && s.t3_cells > 0) return s;  // the shared-memory window was chosen for 128 x 2

@@ -18,9 +18,10 @@ def fresh(engine):
     engine.set_variant(0)
 
 
-# (n, first, count): one particle, one tile, below and above 2.5e7 and 8e9 pairs, short ranges against many particles
+# (n, first, count): one particle, one tile, below and above 3e7, 1.5e8 and 8e9 pairs, short ranges against many particles
 RANGES = [(1, 0, 1), (64, 0, 63), (65, 1, 64), (5001, 0, 4990), (5011, 0, 5005), (100003, 5, 1), (100003, 50000, 33),
-          (120001, 20000, 66000), (120001, 0, 67500)]
+          (120001, 20000, 66000), (120001, 0, 67500), (5475, 0, 5475), (5479, 0, 5479),
+          (12247, 0, 12247), (12248, 0, 12248)]
 
 
 @pytest.mark.parametrize("n,lo,count", RANGES)

@@ -24,9 +24,9 @@ def fresh(engine):
     eng.set_variant(0)
 
 
-@pytest.mark.parametrize("n", [16384, 16385, 16511, 20001, 39999, 40000, 65600, 70001, 99999, 100000, 100353])
+@pytest.mark.parametrize("n", [16384, 16385, 16511, 19999, 20000, 20001, 39999, 40000, 65600, 70001, 99999, 100000, 100353])
 def test_r3_sizes(fresh, n):
-    """Taken from n = 16,384 on; wider rows from 40,000 on, groups of several rows from 32,769 (narrow) and 65,537 on."""
+    """Taken from n = 20,000 on; groups of several rows from 32,769 on, wider rows from 100,000 on."""
     ps = W.r3_compactified(n, 480.0, seed=n, displace=True)
     fresh.set_particles(ps.m, ps.eps)
     p = S.params(S.R3, cosmology=1, comoving=1, mius=1e-3)
@@ -42,16 +42,16 @@ def test_r3_softened_and_coincident(fresh):
     """Pairs inside the spline, a coincident pair, and unsoftened particles beside
     padding (their self pair is 0 * inf in the FP64 kernel, as in the reference)."""
     rng = np.random.default_rng(5)
-    x = rng.normal(0, 0.5, (16500, 3))
+    x = rng.normal(0, 0.5, (20500, 3))
     x[1] = x[0]
-    eps = np.full(16500, 0.1)
-    eps[16400:] = 0.0
-    m = rng.uniform(0.5, 2.0, 16500)
+    eps = np.full(20500, 0.1)
+    eps[20400:] = 0.0
+    m = rng.uniform(0.5, 2.0, 20500)
     fresh.set_particles(m, eps)
     F = fresh.forces(x, S.params(S.R3), S.MIXED)
     F64 = fresh.forces(x, S.params(S.R3), S.FP64)
     ok = np.isfinite(F64).all(1)
-    assert ok[:16400].all() and np.array_equal(np.isfinite(F).all(1), ok)
+    assert ok[:20400].all() and np.array_equal(np.isfinite(F).all(1), ok)
     assert err_stats(F[ok], F64[ok])["p99"] < MIXED_P99
 
 
@@ -59,7 +59,7 @@ def test_r3_softened_and_coincident(fresh):
 def test_r3_units(fresh, scale):
     """Lengths far from 1: r^-3 itself leaves the FP32 range at 1e13, its products with the masses do not; at 1e-9
     those products overflow in the softened core. Nothing the one-sided kernel represents is lost."""
-    ps = W.r3_compactified(16500, 480.0, seed=3, displace=True)
+    ps = W.r3_compactified(20500, 480.0, seed=3, displace=True)
     m = ps.m * 1e10
     fresh.set_particles(m, ps.eps * scale)
     p = S.params(S.R3)
@@ -76,7 +76,7 @@ def test_r3_units(fresh, scale):
 
 def test_r3_kdk_and_choice(fresh):
     """The leapfrog on it, and an explicit pair loop switching it off: the same forces to rounding."""
-    ps = W.r3_compactified(17000, 480.0, seed=11, displace=True)
+    ps = W.r3_compactified(21000, 480.0, seed=11, displace=True)
     p = S.params(S.R3)
     out = []
     for variant in (None, 1):
