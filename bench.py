@@ -59,7 +59,11 @@ UNIT = "pairs/s"
 # (index radius 3), k vectors |k| <= 5 (2 pi / L) (index radius 6).
 T3_NG = 63
 LOOPS = ["fp32", "fp32x2", "fp32x2 (768 threads/SM)", "fp32x2 (1024 threads/SM)", "fp32x2, bulk-copy mbarrier pipeline"]
-# DRAM bytes (read + write) of one launch of the pair kernel, from one-pass ncu
+# Mixed forces of all particles run the pairwise kernels (each pair evaluated
+# once for both particles) from these sizes on, unless a shape is set.
+PAIRWISE_MIN_R3, PAIRWISE_MIN_PERIODIC = 20000, 4096
+PAIRWISE = "pairwise: each pair of particles evaluated once for both"
+# DRAM bytes (read + write) of one launch of a one-sided pair kernel, from one-pass ncu
 # captures of dram__bytes_read.sum + dram__bytes_write.sum, keyed by
 # (workload, N, threads, ipt, pair-loop variant): the traffic is reported only
 # for the shape that was timed, else null.
@@ -487,7 +491,15 @@ def measure(eng, S, ps, p, flops, table, steps, warmup, fp64_sample, f32_peak, f
     }
 
 
-def shape_desc(shape, args):
+def pairwise(args, n):
+    """Whether a force call without a set shape runs a pairwise kernel (the
+    tables of the workloads are odd, as those need; NGP runs one-sided)."""
+    if args.workload in ("cfg2", "cfg3"):
+        return n >= PAIRWISE_MIN_PERIODIC and not (getattr(args, "s1_table", False) and args.order == 0)
+    return n >= PAIRWISE_MIN_R3
+
+
+def shape_desc(shape, args, n=0):
     """The kernel shape; the variant names the R^3 pair loop, or for T^3 with
     a table the lane mapping (the other workloads have one pair loop)."""
     w = getattr(args, "workload", "cfg1")
@@ -500,15 +512,17 @@ def shape_desc(shape, args):
             return "quad lanes" if v == 1 else "one i per lane"
         return "fp32"
 
+    if shape and pairwise(args, n):
+        return PAIRWISE
     if shape:
         return {"threads": shape[0], "ipt": shape[1], "pair_loop": loop(shape[2])}
     return (args.shape or "128x2") + " " + loop(max(args.variant, 0))
 
 
-def traffic_of(workload_name, n, shape):
-    if not shape:
+def traffic_of(args, n, shape, tuned):
+    if not shape or (tuned and pairwise(args, n)):
         return None
-    return NCU_TRAFFIC.get((workload_name, n, shape[0], shape[1], shape[2]))
+    return NCU_TRAFFIC.get((args.workload, n, shape[0], shape[1], shape[2]))
 
 
 def run_ours(args, ws, rank, local, dist):
@@ -565,6 +579,8 @@ def run_ours(args, ws, rank, local, dist):
     nominal, nsm = nominal_fp32_peak(clk.get("sm_mhz"))
     achieved = r["achieved"]
     timed_shape = r["shape"] or shape_used
+    # FMA-pipe instructions per force contribution (R^3)
+    fma_ops = (8 if r["shape"] and pairwise(args, n) else 12) if args.workload in ("cfg0", "cfg1") else None
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": float(np.mean(r["step_ms"])), "higher_is_better": True, "scaling": "weak",
@@ -573,7 +589,7 @@ def run_ours(args, ws, rank, local, dist):
         "config": {"workload": desc + ", one full force evaluation per step", "n": n, "pairs_per_step": pairs_step,
                    "parallelism": "one independent realisation per GPU" if ws > 1 else "1 GPU",
                    "l2": "512 MB flush between steps", "precision": "mixed",
-                   "kernel_shape": shape_desc(r["shape"], args), "prep_ms": r["prep_ms"],
+                   "kernel_shape": shape_desc(r["shape"], args, n), "prep_ms": r["prep_ms"],
                    "autotune_s": r["autotune_s"]},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(x_pin.nbytes),
                 "d2h_bytes_per_step": int(F_host.nbytes), "ms_per_step": e2e_t * 1e3,
@@ -582,14 +598,18 @@ def run_ours(args, ws, rank, local, dist):
                          "ms_per_step": float(np.mean(e2e_pg)) * 1e3,
                          "host_memory": "ordinary malloc'd numpy arrays, as the reference's driver passes x and F"},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": f32_peak / 1e12, "unit": "TFLOP/s",
-                     "frac": r["frac"], "traffic": traffic_of(args.workload, n, timed_shape),
+                     "frac": r["frac"], "traffic": traffic_of(args, n, timed_shape, bool(r["shape"])),
                      "traffic_note": "DRAM bytes of one pair-kernel launch from an ncu capture of the timed shape "
                                      "(null: no capture of this shape); compute-bound",
                      "peak_kind": "FP32 FMA issue peak measured in this process (dependent-FMA-chain kernel); "
                                   "MEASURED_PEAKS.json holds HBM and bf16-tensor figures only",
                      "nominal_peak_at_sampled_clock": nominal, "sms": nsm,
                      "frac_of_nominal": achieved / nominal if nominal else None,
-                     "flops_per_pair": flops, "kernel_ms": r["kernel_ms"]},
+                     "flops_per_pair": flops, "kernel_ms": r["kernel_ms"],
+                     "flops_note": "flop of one force contribution evaluated on its own (value counts these); a "
+                                   "pairwise kernel executes fewer: in R^3 16 FMA-pipe instructions for the two "
+                                   "contributions of a pair, 12 each one-sided",
+                     "fma_pipe_frac": r["kern_rate"] * fma_ops * 2 / f32_peak if fma_ops else None},
         "fp64": r["fp64"],
         "speedup_vs_fp64": r["speedup_vs_fp64"],
         "accuracy_mixed_vs_fp64": r["accuracy"],
@@ -645,7 +665,7 @@ def kdk_measure(eng, S, W, ps, steps, warmup, f32_peak, nkdk=4, dt=1e-3):
     return {"workload": f"R3 compactified N={n} R_max=480 Mpc: one force evaluation + {nkdk} KDK steps at dt={dt} "
                         f"from rest (the workload as specified), mixed and FP64",
             "value": value, "unit": UNIT, "ms_per_step": res["mixed"]["ms_per_step"], "steps": steps,
-            "pairs_per_step": pairs, "kernel_shape": shape_desc(shape, argparse.Namespace(shape="", variant=-1, workload="cfg0")),
+            "pairs_per_step": pairs, "kernel_shape": shape_desc(shape, argparse.Namespace(shape="", variant=-1, workload="cfg0"), ps.n),
             "autotune_s": t_tune,
             "roofline": {"bound": "fp32", "frac_of_step": value * 20 / f32_peak, "peak": f32_peak / 1e12,
                          "flops_per_pair": 20,
@@ -794,7 +814,7 @@ def run_configs(args, eng, peaks, local):
         rate, dt, pairs, ni = cpu_baseline(ps, p, 0, threads, tab, seconds=2.0)
         out[name] = {"workload": desc, "value": r["value"], "unit": UNIT, "ms_per_step": float(np.mean(r["step_ms"])),
                      "steps": len(r["step_ms"]), "kernel_ms": r["kernel_ms"], "prep_ms": r["prep_ms"],
-                     "kernel_pairs_per_s": r["kern_rate"], "kernel_shape": shape_desc(r["shape"], ca),
+                     "kernel_pairs_per_s": r["kern_rate"], "kernel_shape": shape_desc(r["shape"], ca, ps.n),
                      "autotune_s": r["autotune_s"],
                      "roofline": {"bound": "fp32", "frac": r["frac"], "achieved": r["achieved"],
                                   "peak": f32_peak / 1e12, "unit": "TFLOP/s", "flops_per_pair": flops},

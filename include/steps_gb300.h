@@ -218,7 +218,7 @@ int steps_gpu_download_state(double *x, double *v, double *F);
 /* Registers `count` independent R^3 realisations; realisation k has n[k]
  * particles whose positions, masses and softening lengths are the host arrays
  * x[k] (double[3 n[k]]), m[k], eps[k]. Velocities start at zero. Registering
- * the same count and n[] again replaces the data only: the tuned tile shape
+ * the same count and n[] again replaces the data only: the tuned row width
  * and the captured graph of the previous batch are kept. */
 int steps_gpu_batch_set(int count, const int *n, const double *const *x, const double *const *m,
                         const double *const *eps);
@@ -226,11 +226,11 @@ int steps_gpu_batch_set(int count, const int *n, const double *const *x, const d
 /* One force evaluation followed by nsteps fixed-h KDK steps of every
  * realisation (StePS/src/step.cc:100-312 with g = 1, a = 1, no Hubble drag).
  * graph = 1 runs the whole of it as ONE persistent kernel, after a single
- * ordering pass, captured into a CUDA graph: (stage, item) tasks from one
- * queue, each stage of a realisation starting when its previous stage is
- * done (bounded waits: STEPS_E_TIMEOUT if one gives up), the kicks, drift and
- * re-tiling done by the block that completes each tile; tile shape, j-chunk
- * length and grid size autotuned on the first run. graph = 2 runs it as a
+ * ordering pass, captured into a CUDA graph: tasks from one queue that evaluate
+ * each pair of particles once, or add up, kick, drift and re-tile 32 particles,
+ * each stage of a realisation starting when its previous stage is done (bounded
+ * waits: STEPS_E_TIMEOUT if one gives up); row width and item size autotuned on
+ * the first run. graph = 2 runs it as a
  * CUDA graph of per-phase kernels (re-ordering every step); graph = 0 as
  * `count` separate plain launches per phase. */
 int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double h, int graph);
