@@ -230,9 +230,7 @@ __device__ __forceinline__ void far_images(const BoxArgs &a, unsigned flags, con
         rho2[h] = f2_fma(dx[h], dx[h], f2_mul(dy[h], dy[h]));
         sw[h] = sz[h] = 0ull;
     }
-    float fm = (float)(m0 - 64);
-#pragma unroll 1
-    for (int m = m0; m <= m1; m++, fm += 1.0f) {
+    auto image = [&](float fm, bool straddles) {
         const float sh = fm * a.t.L;
         const f2 s2 = f2_bcast(sh);
         f2 dzm[2], w[2];
@@ -244,7 +242,7 @@ __device__ __forceinline__ void far_images(const BoxArgs &a, unsigned flags, con
             const f2 ri = f2_pack(rsqrt_mufu(r0), rsqrt_mufu(r1));
             w[h] = f2_mul(f2_mul(ri, ri), ri);
         }
-        if (m < i0 || m > i1) {  // straddles the cut (warp-uniform)
+        if (straddles) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 float z[2], v[2];
@@ -264,6 +262,22 @@ __device__ __forceinline__ void far_images(const BoxArgs &a, unsigned flags, con
         for (int h = 0; h < 2; h++) {
             sw[h] = f2_add(sw[h], w[h]);
             sz[h] = f2_fma(w[h], dzm[h], sz[h]);
+        }
+    };
+    // The images entirely inside the cut are consecutive; their loop is unrolled
+    // (n = 100,003, one loop for all / this: 7 images 11.5 / 11.2 ms, 31 images
+    // 43.7 / 40.6; unrolled 2, 3 or 6 times up to 3 % slower).
+    int m = m0;
+    float fm = (float)(m0 - 64);
+#pragma unroll 1
+    while (m <= m1) {
+        if (m >= i0 && m <= i1) {
+#pragma unroll 4
+            for (; m <= i1; m++, fm += 1.0f) image(fm, false);
+        } else {
+            image(fm, true);
+            m++;
+            fm += 1.0f;
         }
     }
 }
