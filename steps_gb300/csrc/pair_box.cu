@@ -335,7 +335,12 @@ __device__ __forceinline__ void near_pair(const BoxArgs &a, unsigned flags, cons
     const float rho2 = fmaf(n[0], n[0], n[1] * n[1]), b2 = b * b;
     if (K == B_S1_IMG) {
         float sw = 0.0f, sz = 0.0f;
-        for (int m = -a.t.emax; m <= a.t.emax; m++) {
+        const int m1 = (int)(flags >> 7 & 127u) - 64;
+        // the other images are outside the cut (all 2 emax + 1 in turn: n = 20,000
+        // 0.79 ms, n = 100,003 11.4; this 0.73 and 11.1; not unrolled, 31 images
+        // 2.63 instead of 2.41 ms at n = 20,000)
+#pragma unroll 2
+        for (int m = (int)(flags & 127u) - 64; m <= m1; m++) {
             const float sh = (float)m * a.t.L, dzm = d[2] + sh;
             const float r2 = fmaf(dzm, dzm, rho2);
             const float ri = rsqrt_mufu(r2);
