@@ -23,9 +23,10 @@
 // positions, velocities, slabs) is read through L2.
 //
 // Measured (12 realisations of 4,736 to 65,024 particles, 1 + 4 stages, 6.4e10
-// ordered pairs): whole batch call 35.1 ms with the one-sided kernel that this
-// one replaced, 29.2 with this one; 4.9 ms a stage, 2.6e12 pairs/s, of which the
-// finish tasks are 3 %.
+// ordered pairs): whole batch call with the data 35.2 ms with the one-sided
+// kernel that this one replaced, 27.7 with this one; 4.8 ms a stage, 2.7e12
+// pairs/s, of which the finish tasks are 3 %. Four blocks an SM, as in
+// pair_sym.cu: 24.1 ms for the run against 24.5 with 6 blocks for narrow rows.
 #include <algorithm>
 
 #include "context.cuh"

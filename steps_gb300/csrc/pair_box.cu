@@ -398,7 +398,7 @@ __device__ __forceinline__ float sum_b(const float *v, int b)
 // wide stencils want registers, the others warps (n = 100,001, 3 / 4 / 5 / 6
 // blocks: trilinear 36.7 / 35.8 / 36.8 / 38.8 ms, tricubic 254 / 269 / 275 /
 // 278, CIC 24.6 / 21.3 / 19.8 / 19.2, TSC 42.7 / 45.4 / 47.0 / 48.8, images
-// 12.6 with 4, 11.6 with 5, 12.8 with 6; T^3 nearest image 7.8 / 7.1 / 6.7).
+// 11.6 with 4, 11.2 with 5, 11.5 with 6; T^3 nearest image 7.8 / 7.1 / 6.7).
 constexpr int box_blocks(int K)
 {
     return K == B_T3_CUB || K == B_S1_TSC ? 3 : K == B_T3_LIN ? 4 : K == B_S1_IMG || K == B_S1_NEAR ? 5 : 6;
