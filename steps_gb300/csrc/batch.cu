@@ -275,6 +275,12 @@ void batch_forces(Batch &b)
     note_launch("k_batch_reduce");
 }
 
+// Counters of the persistent kernel: the queue, two per realisation, one per tile.
+size_t ensemble_ctl_bytes(const Batch &b)
+{
+    return sizeof(unsigned long long) * (1 + 2 * (size_t)b.count) + sizeof(unsigned) * b.ntiles;
+}
+
 // The whole run in one persistent kernel (stream-ordered, capturable): one
 // ordering pass, the counters zeroed, then k_ensemble over nsteps + 1 stages.
 void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
@@ -282,13 +288,13 @@ void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
     batch_order(b, false);
-    unsigned *ctl = b.ens_ctl.as<unsigned>();
-    STEPS_CUDA(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * (1 + 2 * (size_t)b.count + b.ntiles), st));
+    unsigned long long *ctl = b.ens_ctl.as<unsigned long long>();
+    STEPS_CUDA(cudaMemsetAsync(ctl, 0, ensemble_ctl_bytes(b), st));
     EnsembleArgs e{};
     e.rel = b.rels.as<EnsRel>();
     e.tasks = b.tasks.as<int4>();
     e.ntasks = b.ens_tasks;
-    e.nstages = nsteps + 1;
+    e.nsteps = nsteps;
     e.nrel = b.count;
     e.pack = b.ts.pack.as<float4>();
     e.resid = b.ts.resid.as<float4>();
@@ -300,7 +306,7 @@ void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
     e.queue = ctl;
     e.pair_done = ctl + 1;
     e.fin_done = ctl + 1 + b.count;
-    e.tile_cnt = ctl + 1 + 2 * b.count;
+    e.tile_cnt = reinterpret_cast<unsigned *>(ctl + 1 + 2 * b.count);
     e.x = b.x.as<double>();
     e.v = b.v.as<double>();
     e.F = b.F.as<double>();
@@ -379,7 +385,7 @@ void ensemble_plan_most(Batch &b, int NP, int split, int most)
     b.ts.resid.ensure<float4>(padded);
     b.ts.sub.ensure<float4>(2 * (padded / SUBTILE));
     b.part.ensure<double>(part);
-    b.ens_ctl.ensure<unsigned>(1 + 2 * (size_t)b.count + b.ntiles);
+    b.ens_ctl.ensure<char>(ensemble_ctl_bytes(b));
     STEPS_CUDA(cudaMemcpyAsync(b.tdesc.ensure<int2>(desc.size()), desc.data(), desc.size() * sizeof(int2),
                                cudaMemcpyHostToDevice, c.stream));
     STEPS_CUDA(cudaMemcpyAsync(b.rels.ensure<EnsRel>(rel.size()), rel.data(), rel.size() * sizeof(EnsRel),

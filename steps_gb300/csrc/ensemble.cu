@@ -42,9 +42,10 @@ using namespace mixed;
 
 // Bounded spin on a counter that other warps increment: true once it reaches
 // target; false after `limit` cycles or as soon as the status word is set.
-__device__ __forceinline__ bool wait_counter(const unsigned *cnt, unsigned target, long long limit, const int *status)
+__device__ __forceinline__ bool wait_counter(const unsigned long long *cnt, unsigned long long target, long long limit,
+                                             const int *status)
 {
-    const volatile unsigned *c = cnt;
+    const volatile unsigned long long *c = cnt;
     const volatile int *st = status;
     if (*c >= target) return true;
     const long long t0 = clock64();
@@ -137,7 +138,7 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
 {
     const int lane = threadIdx.x & 31;
     const EnsRel R = e.rel[k];
-    const bool kick2 = stage >= 1, kick1 = stage < e.nstages - 1;
+    const bool kick2 = stage >= 1, kick1 = stage < e.nsteps;
     const double h2 = e.h / 2.0;
     const double *pi = e.part + R.part, *pj = pi + 3 * (size_t)R.C * R.npad;
     const int q = b * 32 + lane, tile = R.tile0 + (b >> 2);
@@ -181,7 +182,7 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
     if (kick1) rebuild_tile(e, tile);
     __threadfence();
     __syncwarp();
-    if (lane == 0 && !(stage == 0 && k == e.stall_rel)) atomicAdd(e.fin_done + k, 1u);
+    if (lane == 0 && !(stage == 0 && k == e.stall_rel)) atomicAdd(e.fin_done + k, 1ull);
 }
 
 template <int NP>
@@ -191,31 +192,30 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(Ensembl
     __shared__ SymArgs sha[SYM_WARPS];  // each warp's item, out of the pair loop's registers
     const int lane = threadIdx.x & 31;
     SymArgs &a = sha[threadIdx.x >> 5];
-    const int total = e.ntasks * e.nstages;
+    const long long total = (long long)e.ntasks * (e.nsteps + 1LL);
     for (;;) {
-        int task = 0;
+        int stage = -1, which = 0;
         if (lane == 0) {
             const volatile int *st = e.status;
-            task = *st != 0 ? total : (int)atomicAdd(e.queue, 1u);
+            const long long task = *st != 0 ? total : (long long)atomicAdd(e.queue, 1ull);
             if (task < total) {
-                const int stage = task / e.ntasks;
-                const int4 d = __ldg(e.tasks + task % e.ntasks);
+                stage = (int)(task / e.ntasks);
+                which = (int)(task % e.ntasks);
+                const int4 d = __ldg(e.tasks + which);
                 const EnsRel *R = e.rel + d.x;
-                const bool ok = d.w ? wait_counter(e.pair_done + d.x, (unsigned)(__ldg(&R->npair) * (stage + 1)), e.wait_cycles,
-                                                     e.status)
-                                    : wait_counter(e.fin_done + d.x, (unsigned)(__ldg(&R->ntiles) * stage), e.wait_cycles,
-                                                     e.status);
+                const bool ok = d.w ? wait_counter(e.pair_done + d.x, __ldg(&R->npair) * (stage + 1ull), e.wait_cycles, e.status)
+                                    : wait_counter(e.fin_done + d.x, __ldg(&R->ntiles) * (unsigned long long)stage,
+                                                   e.wait_cycles, e.status);
                 if (!ok) {
                     atomicExch(e.status, STEPS_E_TIMEOUT);
-                    task = total;
+                    stage = -1;
                 }
             }
             __threadfence();
         }
-        task = __shfl_sync(0xffffffffu, task, 0);
-        if (task >= total) return;
-        const int stage = task / e.ntasks;
-        const int4 d = __ldg(e.tasks + task % e.ntasks);
+        stage = __shfl_sync(0xffffffffu, stage, 0);
+        if (stage < 0) return;
+        const int4 d = __ldg(e.tasks + __shfl_sync(0xffffffffu, which, 0));
         int k = d.x;
         STEPS_CHECK_IDX(k, e.nrel, CK_I_TILE);
         if (d.w) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(Ensembl
             sym_item<NP, true>(a, shw[threadIdx.x >> 5], d.y, d.z);
             __threadfence();
             __syncwarp();
-            if (lane == 0) atomicAdd(e.pair_done + k, 1u);
+            if (lane == 0) atomicAdd(e.pair_done + k, 1ull);
         }
     }
 }

@@ -20,14 +20,16 @@ struct EnsRel {
 struct EnsembleArgs {
     const EnsRel *rel;
     const int4 *tasks;      // of one stage: (realisation, group, chunk, 0) or (realisation, 32 particles, 0, 1)
-    int ntasks, nstages, nrel;
+    int ntasks, nsteps, nrel;  // nsteps + 1 stages
     float4 *pack, *resid, *meta, *sub;
     const float *eps;       // softening (constant over the run)
     const uint32_t *idx;    // original index of each padded position (constant)
     double *part;
-    unsigned *queue;        // task counter
-    unsigned *pair_done, *fin_done;  // per realisation: items, tiles done, over all stages
-    unsigned *tile_cnt;     // per tile: finish tasks done, over all stages
+    // 64 bits: a stage of 64 realisations of 8,192 particles is up to 242,000
+    // tasks, 2^31 of them fewer than 9,000 steps.
+    unsigned long long *queue;                 // task counter, over all stages
+    unsigned long long *pair_done, *fin_done;  // per realisation: items, tiles done, over all stages
+    unsigned *tile_cnt;     // per tile: finish tasks done, over all stages, modulo 2^32 (read modulo 4)
     double *x, *v, *F;      // caller-order FP64 positions, velocities, forces
     double h;               // fixed step; acceleration g F a^-3 - 2 H v with g = 1, a = 1, H = 0
     float guard2;
