@@ -283,7 +283,7 @@ size_t ensemble_ctl_bytes(const Batch &b)
 
 // The whole run in one persistent kernel (stream-ordered, capturable): one
 // ordering pass, the counters zeroed, then k_ensemble over nsteps + 1 stages.
-void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
+void ensemble_run(Batch &b, int nsteps, double h, int stall_rel, bool hold = false)
 {
     Ctx &c = ctx();
     cudaStream_t st = c.stream;
@@ -311,6 +311,7 @@ void ensemble_run(Batch &b, int nsteps, double h, int stall_rel)
     e.v = b.v.as<double>();
     e.F = b.F.as<double>();
     e.h = h;
+    e.hold = hold;
     e.guard2 = c.shape.guard * c.shape.guard;
     e.n = b.ntot;
     e.ntiles = b.ntiles;
@@ -410,9 +411,11 @@ void ensemble_plan(Batch &b, int NP, int split)
     }
 }
 
-// Times three stages (two steps of length 0, which leave positions and velocities
-// as they are) per row width and item size, and keeps the fastest: one stage
-// alone overrates small items, which end evenly but cost more slabs.
+// Times three stages per row width and item size, and keeps the fastest: one
+// stage alone overrates small items, which end evenly but cost more slabs.
+// Positions and velocities are not written: steps of length 0 would leave finite
+// ones as they are, but turn those of a particle whose force is infinite or NaN
+// into NaN.
 void ensemble_tune(Batch &b)
 {
     Ctx &c = ctx();
@@ -422,9 +425,9 @@ void ensemble_tune(Batch &b)
     for (int np = 2; np <= 4; np += 2)
         for (int sp : splits) {
             ensemble_plan(b, np, sp);
-            ensemble_run(b, 0, 0.0, -1);  // warm
+            ensemble_run(b, 0, 0.0, -1, true);  // warm
             STEPS_CUDA(cudaEventRecord(c.marks[12], c.stream));
-            ensemble_run(b, 2, 0.0, -1);
+            ensemble_run(b, 2, 0.0, -1, true);
             STEPS_CUDA(cudaEventRecord(c.marks[13], c.stream));
             STEPS_CUDA(cudaEventSynchronize(c.marks[13]));
             float ms = 0;

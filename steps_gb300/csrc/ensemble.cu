@@ -164,6 +164,7 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
         for (int c = 0; c < 3; c++) {
             const size_t p = 3 * (size_t)o + c;
             e.F[p] = f[c];
+            if (e.hold) continue;
             double vv = __ldcg(e.v + p);
             // acceleration g F a^-3 - 2 H v at g = 1, a = 1, H = 0, as the batch's KDK kernels evaluate it
             if (kick2) vv += (1.0 * f[c] * 1.0 - 2.0 * 0.0 * vv) * h2;

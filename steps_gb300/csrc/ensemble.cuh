@@ -31,6 +31,7 @@ struct EnsembleArgs {
     unsigned long long *pair_done, *fin_done;  // per realisation: items, tiles done, over all stages
     unsigned *tile_cnt;     // per tile: finish tasks done, over all stages, modulo 2^32 (read modulo 4)
     double *x, *v, *F;      // caller-order FP64 positions, velocities, forces
+    bool hold;              // stages are evaluated and tiles rebuilt, x and v left as they are (timing)
     double h;               // fixed step; acceleration g F a^-3 - 2 H v with g = 1, a = 1, H = 0
     float guard2;
     int n, ntiles;

@@ -3,6 +3,8 @@ import numpy as np
 import pytest
 
 import steps_gb300 as S
+from helpers import err_stats
+from steps_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +31,21 @@ def test_more_tasks_than_an_int(engine):
     assert abs((1.0 - (x[1, 0] - x[0, 0])) / (1.0 - d) - 1.0) < 1e-6
     assert abs((v[1, 0] - v[0, 0]) / w - 1.0) < 1e-6
     assert abs(F[0, 0] / (-0.5 * a) - 1.0) < 1e-6
+
+
+@pytest.mark.parametrize("graph", [1, 2])
+def test_tuning_leaves_the_state(engine, graph):
+    """The first run times candidate shapes on the registered data. An unsoftened particle's self pair is 0 * inf, so its
+    force is NaN, in every path; nothing else may be: not its position or velocity, nor the others' forces."""
+    sets = [W.r3_compactified(n, 300.0, seed=n, displace=True) for n in (300, 700)]
+    sets[0].eps[5] = 0.0
+    engine.batch_set([s.x for s in sets], [s.m for s in sets], [s.eps for s in sets])
+    engine.batch_run(S.params(S.R3), S.MIXED, 0, 1e-3, graph=graph)
+    for k, s in enumerate(sets):
+        x, v, F = engine.batch_get(k)
+        assert np.array_equal(x, s.x) and not v.any()
+        good = np.ones(len(F), bool)
+        good[5] = k != 0
+        assert np.array_equal(np.isfinite(F).all(1), good)
+        engine.set_particles(s.m, s.eps)
+        assert err_stats(F[good], engine.forces(s.x, S.params(S.R3), S.FP64)[good])["p99"] < 1e-5
