@@ -61,6 +61,7 @@ struct Batch {
     cudaGraphExec_t exec = nullptr;
     int graph_steps = -1, graph_mode = 0;
     double graph_h = 0.0;
+    float graph_guard = 0.0f;  // the precision guard, a constant of the captured kernels
 };
 
 namespace {
@@ -660,7 +661,8 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
                 b.tuned = true;
                 release_graph(b);
             }
-            if (!b.exec || b.graph_steps != a.nsteps || b.graph_h != a.h || b.graph_mode != a.graph) {
+            if (!b.exec || b.graph_steps != a.nsteps || b.graph_h != a.h || b.graph_mode != a.graph ||
+                b.graph_guard != c.shape.guard) {
                 release_graph(b);
                 // the plan of the chosen path (the two paths keep their own shapes)
                 if (persistent) ensemble_plan(b, b.ens_np, b.ens_split);
@@ -687,6 +689,7 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
                 b.graph_steps = a.nsteps;
                 b.graph_h = a.h;
                 b.graph_mode = a.graph;
+                b.graph_guard = c.shape.guard;
             }
             STEPS_CUDA(cudaGraphLaunch(b.exec, c.stream));
             add_launches(b.graph_kernels);  // the kernels the graph runs

@@ -49,3 +49,26 @@ def test_tuning_leaves_the_state(engine, graph):
         assert np.array_equal(np.isfinite(F).all(1), good)
         engine.set_particles(s.m, s.eps)
         assert err_stats(F[good], engine.forces(s.x, S.params(S.R3), S.FP64)[good])["p99"] < 1e-5
+
+
+@pytest.mark.parametrize("graph", [1, 2])
+def test_precision_guard_between_runs(engine, graph):
+    """A captured run is captured again when the precision guard changes: its forces are those of a run that had to be
+    captured under the new guard (one of another length came between), and of the old guard once that is back."""
+    sets = [W.r3_compactified(n, 300.0, seed=n, displace=True) for n in (3000, 900)]
+    p = S.params(S.R3)
+
+    def run(guard, steps=0):
+        engine.set_guard(guard)
+        engine.batch_set([s.x for s in sets], [s.m for s in sets], [s.eps for s in sets])
+        engine.batch_run(p, S.MIXED, steps, 1e-3, graph=graph)
+        return np.concatenate([engine.batch_get(k)[2] for k in range(len(sets))])
+
+    try:
+        before, fine = run(30.0), run(2.0)
+        run(2.0, steps=1)
+        assert np.array_equal(fine, run(2.0))
+        assert not np.array_equal(fine, before)
+        assert np.array_equal(before, run(30.0))
+    finally:
+        engine.set_guard(30.0)
