@@ -607,20 +607,22 @@ __global__ void k_table_parity(const double *__restrict__ t, long long ncell, in
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double odd = 0.0, big = 0.0;
     if (c < ncell) {
+        bool bad = false;  // fmax drops NaN
         if (nz == 0) {
             for (int k = 0; k < 3; k++) {
                 const double v = t[3 * c + k];
                 odd = fmax(odd, fabs(v + t[3 * (ncell - 1 - c) + k]));
                 big = fmax(big, fabs(v));
-                if (!(v == v)) odd = big = v;
+                bad = bad || !(v == v);
             }
         } else {
             const long long m = c - c % nz + (nz - 1 - c % nz);
             const double dr = t[2 * c], dz = t[2 * c + 1];
             odd = fmax(fabs(dr - t[2 * m]), fabs(dz + t[2 * m + 1]));
             big = fmax(fabs(dr), fabs(dz));
-            if (!(dr == dr) || !(dz == dz)) odd = big = dr + dz;
+            bad = !(dr == dr) || !(dz == dz);
         }
+        if (bad) odd = big = __longlong_as_double(0x7ff8000000000000LL);
     }
     // bit patterns of non-negative doubles order as integers; NaN above all
     const unsigned long long ob = (unsigned long long)__double_as_longlong(fabs(odd)),

@@ -183,6 +183,28 @@ def test_tables_that_are_not_odd(fresh, topology):
     assert np.array_equal(F, fresh.forces(ps.x, p, S.MIXED))
 
 
+@pytest.mark.parametrize("precision", [S.MIXED, S.FP64])
+@pytest.mark.parametrize("kind,entry", [("t32", 0), ("t32", 1), ("t34", 0), ("t34", 2), ("s1tab2", 0), ("s1tab2", 1)])
+def test_tables_with_a_nan(fresh, kind, entry, precision):
+    """One NaN in one component: only the particles whose own stencils read it get NaN, as one-sided."""
+    n = 4500
+    ps, p = periodic(fresh, kind, n)
+    if kind.startswith("t3"):
+        table = fresh.get_table_t3(31)
+        table[3 * (31 * 31 * 9 + 31 * 14 + 20) + entry] = np.nan
+        fresh.set_table_t3(table, 31)
+    else:
+        table = fresh.get_table_s1r2(432, 64)
+        table[2 * (100 * 64 + 40) + entry] = np.nan
+        fresh.set_table_s1r2(table, 432, 64)
+    fresh.set_particles(ps.m, ps.eps)
+    F = fresh.forces(ps.x, p, precision)
+    half = np.concatenate([fresh.forces(ps.x, p, precision, 0, n // 2), fresh.forces(ps.x, p, precision, n // 2 + 1, n - 1)])
+    bad = np.isnan(half)
+    assert bad.any() and not bad.all()
+    assert np.array_equal(np.isnan(F), bad)
+
+
 # ---- FP64 -----------------------------------------------------------------------
 
 
