@@ -601,34 +601,57 @@ __global__ void __launch_bounds__(SYM_THREADS, box_blocks(K)) k_sym_box(BoxArgs 
 }  // namespace
 
 // Largest |T(c) + T(mirror of c)| and |T(c)| of the T^3 table, or for the
-// (rho, z) table of D_rho(z) - D_rho(-z) and D_z(z) + D_z(-z).
-__global__ void k_table_parity(const double *__restrict__ t, long long ncell, int nz, unsigned long long *out)
+// (rho, z) table of D_rho(z) - D_rho(-z) and D_z(z) + D_z(-z). Bit patterns of
+// magnitudes order as integers, NaN above all. A thread takes a cell and its
+// mirror at a time and a block ends with one atomic per word: the first call
+// after an upload waits for this kernel, and with two atomics per cell on the
+// same two words it took 2.6 ms at Ng = 127 and 21 ms at 255 (with the copy and the wait; now 0.04
+// and 0.22).
+constexpr int PARITY_THREADS = 256;
+__device__ __forceinline__ unsigned long long magnitude_bits(double v)
 {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double odd = 0.0, big = 0.0;
-    if (c < ncell) {
-        bool bad = false;  // fmax drops NaN
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL;
+}
+
+__global__ void __launch_bounds__(PARITY_THREADS) k_table_parity(const double *__restrict__ t, long long ncell, int nz,
+                                                                unsigned long long *out)
+{
+    unsigned long long odd = 0, big = 0;
+    const int half = nz ? (nz + 1) / 2 : 0;
+    const long long npair = nz ? ncell / nz * half : (ncell + 1) / 2;
+    for (long long q = (long long)blockIdx.x * PARITY_THREADS + threadIdx.x; q < npair;
+         q += (long long)gridDim.x * PARITY_THREADS) {
         if (nz == 0) {
+            const double *a = t + 3 * q, *b = t + 3 * (ncell - 1 - q);
+#pragma unroll
             for (int k = 0; k < 3; k++) {
-                const double v = t[3 * c + k];
-                odd = fmax(odd, fabs(v + t[3 * (ncell - 1 - c) + k]));
-                big = fmax(big, fabs(v));
-                bad = bad || !(v == v);
+                odd = max(odd, magnitude_bits(a[k] + b[k]));
+                big = max(big, max(magnitude_bits(a[k]), magnitude_bits(b[k])));
             }
         } else {
-            const long long m = c - c % nz + (nz - 1 - c % nz);
-            const double dr = t[2 * c], dz = t[2 * c + 1];
-            odd = fmax(fabs(dr - t[2 * m]), fabs(dz + t[2 * m + 1]));
-            big = fmax(fabs(dr), fabs(dz));
-            bad = !(dr == dr) || !(dz == dz);
+            const long long row = q / half * nz;
+            const int z = (int)(q % half);
+            const double *a = t + 2 * (row + z), *b = t + 2 * (row + nz - 1 - z);
+            odd = max(odd, max(magnitude_bits(a[0] - b[0]), magnitude_bits(a[1] + b[1])));
+#pragma unroll
+            for (int k = 0; k < 2; k++) big = max(big, max(magnitude_bits(a[k]), magnitude_bits(b[k])));
         }
-        if (bad) odd = big = __longlong_as_double(0x7ff8000000000000LL);
     }
-    // bit patterns of non-negative doubles order as integers; NaN above all
-    const unsigned long long ob = (unsigned long long)__double_as_longlong(fabs(odd)),
-                             bb = (unsigned long long)__double_as_longlong(fabs(big));
-    atomicMax(&out[0], ob);
-    atomicMax(&out[1], bb);
+    __shared__ unsigned long long red[2][PARITY_THREADS / 32];
+    for (int o = 16; o > 0; o >>= 1) {
+        odd = max(odd, __shfl_xor_sync(0xffffffffu, odd, o));
+        big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = odd;
+        red[1][threadIdx.x >> 5] = big;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long m = 0;
+        for (int w = 0; w < PARITY_THREADS / 32; w++) m = max(m, red[threadIdx.x][w]);
+        atomicMax(&out[threadIdx.x], m);
+    }
 }
 
 // Largest asymmetry of a table over its largest entry (NaN: not comparable).
@@ -637,7 +660,8 @@ static double asymmetry(const double *t, long long ncell, int nz)
     Ctx &c = ctx();
     unsigned long long *d = c.bbox.ensure<unsigned long long>(8), h[2];
     STEPS_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof *d, c.stream));
-    k_table_parity<<<(unsigned)((ncell + 255) / 256), 256, 0, c.stream>>>(t, ncell, nz, d);
+    const long long blocks = std::min((ncell + PARITY_THREADS - 1) / PARITY_THREADS, 8LL * c.nsm);
+    k_table_parity<<<(unsigned)blocks, PARITY_THREADS, 0, c.stream>>>(t, ncell, nz, d);
     note_launch("k_table_parity");
     STEPS_CUDA(cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, c.stream));
     STEPS_CUDA(cudaStreamSynchronize(c.stream));

@@ -1,6 +1,7 @@
 """The pairwise kernels (each pair of particles evaluated once, added to both)
 against the FP64 kernels, at the edges of tiles, rows, row widths and groups."""
 import math
+import time
 
 import numpy as np
 import pytest
@@ -203,6 +204,28 @@ def test_tables_with_a_nan(fresh, kind, entry, precision):
     bad = np.isnan(half)
     assert bad.any() and not bad.all()
     assert np.array_equal(np.isnan(F), bad)
+
+
+@pytest.mark.parametrize("ng", [127, 255])
+def test_first_call_after_a_table(fresh, ng):
+    """The first call with a new table looks whether it is odd: one pass over it (50 and 400 MB, 10 and 60 us at the
+    memory's rate) and one wait for the answer, so 0.5 ms more than a later call at most."""
+    ps = W.t3_clumpy(1000, L3, 1)
+    fresh.build_table_t3(ng, L3, 2.0 / L3, 2.0, 5.0 * 2.0 * math.pi / L3, 3.0, 6.0)
+    table = fresh.get_table_t3(ng)
+    p = S.params(S.T3, is_periodic=2, L=L3, rsim=L3 / 2, ewald_order=2)
+    fresh.set_particles(ps.m, ps.eps)
+
+    def call():
+        t0 = time.perf_counter()
+        fresh.forces(ps.x, p, S.FP64)
+        return time.perf_counter() - t0
+
+    first = []
+    for _ in range(4):
+        fresh.set_table_t3(table, ng)
+        first.append(call())
+    assert min(first) - min(call() for _ in range(4)) < 0.5e-3
 
 
 # ---- FP64 -----------------------------------------------------------------------
