@@ -249,20 +249,6 @@ __device__ __forceinline__ float rcp_mufu(float x)
     return y;
 }
 
-// FP64 1/sqrt(x) for 1e-36 < x < 1e36: a single-precision MUFU seed (relative
-// error e0 < 2^-22) refined by one third-order Householder step of Newton's
-// iteration for f(y) = y^-2 - x, i.e. the binomial series of (1 - e)^(-1/2):
-//   e = 1 - x y^2,  y' = y (1 + e/2 + 3 e^2 / 8),  error O(e0^3) < 1e-19,
-// so the result is within a couple of ulp of 1/sqrt(x).
-__device__ __forceinline__ double rsqrt_fp64(double x)
-{
-    double y = (double)rsqrt_mufu(__double2float_rn(x));
-    double t = x * y;
-    double e = fma(-t, y, 1.0);
-    double p = fma(0.375, e, 0.5);
-    return fma(y * e, p, y);
-}
-
 // r^-3 of a pair known to be outside its softening support, from r^2, on as few
 // FP64 instructions as it takes (4). The FP64 pipe, 1/64 of the FP32 rate,
 // bounds the FP64 kernels, so what other pipes can do exactly or accurately
@@ -274,9 +260,9 @@ __device__ __forceinline__ double rsqrt_fp64(double x)
 //   * 15 e^2 / 8 < 2^-40.8 is needed to 2^-13 of itself: FP32.
 // b2: an FP32 upper bound of the squared support. False, with w untouched,
 // where r^2 may lie inside it or outside the FP32 range: the caller then takes
-// softening_fp64. Against the 10 instructions of rsqrt_fp64, its conversions
-// and cube, and 3 for the comparison: R^3 at n = 32,768, one-sided 43.7 -> 31.1
-// ms (with 6 instructions here).
+// softening_fp64. Against a reciprocal root of 10 instructions with its
+// conversions and cube, and 3 for the comparison: R^3 at n = 32,768, one-sided
+// 43.7 -> 31.1 ms (with 6 instructions here).
 __device__ __forceinline__ double widen_fp32(int bits)  // a normal, positive float
 {
     return __hiloint2double((bits >> 3) + (896 << 20), bits << 29);
@@ -326,10 +312,12 @@ __device__ __forceinline__ double spline_inner_fp64(double r, double beta)
     return ib3 * (u * (u * (-32.0 / 3.0 * u + 38.4) - 48.0) + 64.0 / 3.0) - (1.0 / 15.0) / r3;
 }
 
+// Any r^2: few pairs come here (far_r3_fp64), those whose r^2 is outside the
+// FP32 range among them.
 __device__ __forceinline__ double softening_fp64(double r2, double beta)
 {
     if (r2 >= beta * beta) {
-        double y = rsqrt_fp64(r2);
+        const double y = 1.0 / sqrt(r2);
         return y * y * y;
     }
     return spline_inner_fp64(sqrt(r2), beta);

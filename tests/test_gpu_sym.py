@@ -262,3 +262,37 @@ def test_fp64_softened_and_far_units(fresh, port):
         F = fresh.forces(x * scale, S.params(S.R3), S.FP64)
         Fo = port.forces(port.system(0, m, eps * scale, port_params(O)), x * scale)
         assert rel_err(F, Fo).max() < 1e-11, scale
+
+
+@pytest.mark.parametrize("entry", ["forces", "ranges", "noalloc"])
+@pytest.mark.parametrize("scale", [1e-21, 1e-18, 3e18, 1e22])
+def test_fp64_outside_the_fp32_range(fresh, port, scale, entry):
+    """Lengths where r^2 is far below or above what FP32 holds (1.2e-38 to 3.4e38), or partly so; one pair in a hundred
+    or so is softened."""
+    import ctypes as C
+    import pyoracle as O
+    from helpers import port_params
+    rng = np.random.default_rng(6)
+    n = 600
+    x = rng.normal(0, 1.0, (n, 3)) * scale
+    m, eps = rng.uniform(0.5, 2.0, n), np.full(n, 0.1 * scale)
+    p = S.params(S.R3)
+    fresh.set_particles(m, eps)
+    if entry == "forces":
+        F = fresh.forces(x, p, S.FP64)
+    elif entry == "ranges":
+        F = np.concatenate([fresh.forces(x, p, S.FP64, 0, 299), fresh.forces(x, p, S.FP64, 300, n - 1)])
+    else:
+        torch = pytest.importorskip("torch")
+        dx, dm, de = (torch.from_numpy(a).to("cuda") for a in (x, m, eps))
+        dF = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        fn = fresh.lib.steps_gpu_forces_fp64_noalloc
+        fn.argtypes = [C.POINTER(S.Params), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int,
+                       C.c_void_p]
+        assert fn(C.byref(p), dx.data_ptr(), dm.data_ptr(), de.data_ptr(), n, dF.data_ptr(), 0, n - 1, None) == S.STEPS_OK
+        torch.cuda.synchronize()
+        F = dF.cpu().numpy()
+    Fo = port.forces(port.system(0, m, eps, port_params(O)), x)
+    # FP64 sums of 600 terms: about 600 roundings of 1.1e-16 of the sum of magnitudes, which cancels to 1e-2 at worst
+    assert rel_err(F, Fo).max() < 1e-11
