@@ -510,8 +510,11 @@ bool mixed_supported(const KParams &kp) { return select_kernel(kp, 128, 2) != nu
 // 1892; 66,667 x 200,003 7401 with 128 x 2 scalar, 5600 packed). Periodic:
 // 64 x 1, whose smaller boxes send fewer pairs down the near path (33,333 x
 // 100,000, ms, 128 x 2 -> 64 x 1: trilinear 34.0 -> 29.3, images 17.8 -> 8.8,
-// nearest image 6.1 -> 3.7); from 1e9 pairs on 256 x 1 for the wide stencils,
-// which re-read the table less (tricubic 250 -> 192, CIC 13.2 -> 11.7).
+// nearest image 6.1 -> 3.7); 256 x 1 for the wide stencils of larger calls, which
+// re-read the table less: tricubic from 1e8 pairs on (64 x 1 / 256 x 1, ms: 4,000
+// x 12,000 6.42 / 6.74; 8,000 x 20,000 18.8 / 17.4; 13,334 x 40,000 56.0 / 47.2;
+// 20,000 x 60,000 118.6 / 95.7), CIC and TSC, which differ less (20,000 x 40,000
+// 3.28 / 3.26 and 8.47 / 8.38; CIC at 3.3e9 pairs 13.2 / 11.7), from 1e9.
 Shape auto_shape(const KParams &kp, int ni, int n)
 {
     Shape s = ctx().shape;
@@ -524,8 +527,9 @@ Shape auto_shape(const KParams &kp, int ni, int n)
     }
     if (kp.topology == STEPS_T3 && s.t3_cells > 0) return s;  // the shared-memory window was chosen for 128 x 2
     const bool s1tab = kp.topology == STEPS_S1R2 && kp.is_periodic >= 2 && !kp.s1r2_images;
-    const bool wide = kp.topology == STEPS_T3 ? kp.is_periodic >= 2 && kp.order == 4 : s1tab && kp.order != 0;
-    s.threads = wide && pairs >= 1e9 ? 256 : 64;
+    const bool tricubic = kp.topology == STEPS_T3 && kp.is_periodic >= 2 && kp.order == 4;
+    const bool wide = tricubic || (s1tab && kp.order != 0);
+    s.threads = wide && pairs >= (tricubic ? 1e8 : 1e9) ? 256 : 64;
     s.ipt = 1;
     return s;
 }

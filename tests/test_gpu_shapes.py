@@ -84,3 +84,17 @@ def test_periodic(fresh, kind, n, lo, count):
     F = fresh.forces(ps.x, p, S.MIXED, lo, lo + count - 1)
     k = min(count, 300)
     assert err_stats(F[-k:], fresh.forces(ps.x, p, S.FP64, lo + count - k, lo + count - 1))["p99"] < 1e-5
+
+
+@pytest.mark.parametrize("count", [9890, 9910])
+def test_tricubic_line(fresh, count):
+    """Tricubic ranges change shape at 1e8 pairs."""
+    n = 10100  # 1e8 pairs lie between the two counts
+    ps, p = W.t3_clumpy(n, 100.0, 3), S.params(S.T3, is_periodic=2, L=100.0, rsim=50.0, ewald_order=4)
+    fresh.build_table_t3(31, 100.0, 0.02, 2.0, 0.3, 3.0, 6.0)
+    fresh.set_particles(ps.m, ps.eps)
+    lo = n - count
+    F = fresh.forces(ps.x, p, S.MIXED, lo, n - 1)
+    assert err_stats(F[-300:], fresh.forces(ps.x, p, S.FP64, n - 300, n - 1))["p99"] < 1e-5
+    fresh.set_tuning(64 if count * n < 1e8 else 256, 1, 0)
+    assert (F == fresh.forces(ps.x, p, S.MIXED, lo, n - 1)).all()
