@@ -218,7 +218,7 @@ int steps_gpu_download_state(double *x, double *v, double *F);
 /* Registers `count` independent R^3 realisations; realisation k has n[k]
  * particles whose positions, masses and softening lengths are the host arrays
  * x[k] (double[3 n[k]]), m[k], eps[k]. Velocities start at zero. Registering
- * the same count and n[] again replaces the data only: the tuned row width
+ * the same count and n[] again replaces the data only: the tuned item size
  * and the captured graph of the previous batch are kept. */
 int steps_gpu_batch_set(int count, const int *n, const double *const *x, const double *const *m,
                         const double *const *eps);
@@ -229,9 +229,8 @@ int steps_gpu_batch_set(int count, const int *n, const double *const *x, const d
  * ordering pass, captured into a CUDA graph: tasks from one queue that evaluate
  * each pair of particles once, or add up, kick, drift and re-tile 32 particles,
  * each stage of a realisation starting when its previous stage is done (bounded
- * waits: STEPS_E_TIMEOUT if one gives up); row width and item size autotuned on
- * the first run. graph = 2 runs it as a
- * CUDA graph of per-phase kernels (re-ordering every step); graph = 0 as
+ * waits: STEPS_E_TIMEOUT if one gives up); item size autotuned on the first run.
+ * graph = 2 runs it as a CUDA graph of per-phase kernels (re-ordering every step); graph = 0 as
  * `count` separate plain launches per phase. */
 int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double h, int graph);
 

@@ -11,8 +11,8 @@
 // graph = 1: the whole run in ONE persistent kernel (ensemble.cu) after a
 // single ordering pass, captured into a CUDA graph and replayed: pair and finish
 // tasks of all realisations and stages from one queue, bounded waits between the
-// stages of a realisation. The row width and the size of the pair items are
-// chosen by timing candidates first.
+// stages of a realisation. The size of the pair items is chosen by timing
+// candidates first.
 // graph = 2: the same run as a CUDA graph of per-phase kernels (per step:
 // kick+drift, re-order, re-tile, work-list force, reduction, kick).
 // Its work list of items (i tile, j tile range, partial slot), ordered by
@@ -50,10 +50,10 @@ struct Batch {
     long long graph_kernels = 0;
     int nmax = 0;  // largest realisation
     bool tuned = false;     // per-phase graph shape
-    bool ens_tuned = false; // persistent kernel: row width and item size
+    bool ens_tuned = false; // persistent kernel: item size
     int threads_pp = 128, ipt_pp = 2;  // per-phase graph shape
     // persistent path
-    int ens_np = 2, ens_split = 16;
+    int ens_split = 16;
     double ens_wait = 1.0;  // seconds a stage wait may last
     int ens_tasks = 0;
     DevBuf rels, tasks, ens_ctl;
@@ -319,35 +319,31 @@ void ensemble_run(Batch &b, int nsteps, double h, int stall_rel, bool hold = fal
     e.status = kernel_status_word();
     e.stall_rel = stall_rel;
     e.wait_cycles = (long long)(b.ens_wait * (double)mixed::MBAR_WAIT_CYCLES);
-    ensemble_launch(b.ens_np, e, st);
+    ensemble_launch(e, st);
     c.status_pending = true;
 }
 
-// Plans the persistent kernel for rows of 64 NP particles: tiles padded to whole
-// rows, and pair items so large that a stage has about `split` of them per
-// resident warp, at most `most` groups and chunks to a realisation (their number
-// sets the slabs).
-void ensemble_plan_most(Batch &b, int NP, int split, int most)
+// Plans the persistent kernel: pair items so large that a stage has about
+// `split` of them per resident warp, at most `most` groups and chunks to a
+// realisation (their number sets the slabs). A row is a tile.
+void ensemble_plan_most(Batch &b, int split, int most)
 {
     Ctx &c = ctx();
-    const int gran = SYM_HALF * NP, rt = NP / 2;  // particles and tiles of a row
     std::vector<int2> desc;
     std::vector<EnsRel> rel(b.count);
-    double units = 0.0, longest = 0.0;  // (row, tile) pairs, in all and of the largest item
+    double units = 0.0, longest = 0.0;  // tile pairs, in all and of the largest item
     for (int k = 0; k < b.count; k++) {
         EnsRel &R = rel[k];
         R = EnsRel{};
         R.tile0 = (int)desc.size();
         R.ntiles = div_up(b.n[k], SYM_T);
-        R.nrows = div_up(R.ntiles, rt);
-        R.gran = gran;
-        for (int t = 0; t < R.nrows * rt; t++)
-            desc.push_back(make_int2(b.off[k] + std::min(t * SYM_T, b.n[k]), std::max(0, std::min(SYM_T, b.n[k] - t * SYM_T))));
-        R.npad = (size_t)R.nrows * gran;
-        units += 0.5 * R.nrows * (double)R.ntiles;
+        for (int t = 0; t < R.ntiles; t++)
+            desc.push_back(make_int2(b.off[k] + t * SYM_T, std::min(SYM_T, b.n[k] - t * SYM_T)));
+        R.npad = (size_t)R.ntiles * SYM_T;
+        units += 0.5 * R.ntiles * (double)R.ntiles;
     }
-    const double warps = (double)c.nsm * ensemble_blocks(NP) * SYM_WARPS;
-    const double area = std::max(1.0, units / (warps * split));  // (row, tile) pairs of an item
+    const double warps = (double)c.nsm * ensemble_blocks() * SYM_WARPS;
+    const double side = std::sqrt(std::max(1.0, units / (warps * split)));  // of an item, in tiles
     std::vector<int> order(b.count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b.n[x] > b.n[y]; });
@@ -355,13 +351,12 @@ void ensemble_plan_most(Batch &b, int NP, int split, int most)
     std::vector<int4> tasks;
     for (int k : order) {
         EnsRel &R = rel[k];
-        const double side = std::sqrt(area * rt);  // tiles
-        R.G = std::max(div_up(R.nrows, most), (int)std::lround(side / rt));
-        R.G = std::min(std::max(R.G, 1), R.nrows);
+        R.G = std::max(div_up(R.ntiles, most), (int)std::lround(side));
+        R.G = std::min(std::max(R.G, 1), R.ntiles);
         R.C = std::max(1, std::min(std::min(most, R.ntiles), (int)std::lround(R.ntiles / side)));
-        R.step = gran * R.G;
+        R.step = SYM_T * R.G;
         longest = std::max(longest, (double)R.G * div_up(R.ntiles, R.C));
-        const int groups = div_up(R.nrows, R.G);
+        const int groups = div_up(R.ntiles, R.G);
         R.npair = groups * R.C;
         R.part = part;
         part += 3 * ((size_t)R.C * R.npad + sym_slab(groups, R.step, 1, R.npad));
@@ -373,12 +368,11 @@ void ensemble_plan_most(Batch &b, int NP, int split, int most)
     b.ens_tasks = (int)tasks.size();
     b.ntiles = (int)desc.size();
     b.T = SYM_T;
-    b.ens_np = NP;
     b.ens_split = split;
     // A stage wait lasts as long as a pair item at most, when all goes well: a
     // warp evaluates 3e8 pairs a second beside its neighbours (bound: a second,
     // or 8 times that).
-    b.ens_wait = std::max(1.0, 8.0 * longest * gran * SYM_T / 3e8);
+    b.ens_wait = std::max(1.0, 8.0 * longest * SYM_T * SYM_T / 3e8);
     const size_t padded = (size_t)b.ntiles * SYM_T;
     b.ts.pack.ensure<float4>(padded);
     b.ts.eps.ensure<float>(padded);
@@ -398,12 +392,12 @@ void ensemble_plan_most(Batch &b, int NP, int split, int most)
 }
 
 // The same with the slabs within 16 GiB, or less where that does not fit.
-void ensemble_plan(Batch &b, int NP, int split)
+void ensemble_plan(Batch &b, int split)
 {
     int most = (int)std::min(128.0, std::max(4.0, (double)(16LL << 30) / (24.0 * b.ntot) / 1.5));
     for (;;) {
         try {
-            ensemble_plan_most(b, NP, split, most);
+            ensemble_plan_most(b, split, most);
             return;
         } catch (const Error &e) {
             if (e.code != STEPS_E_NOMEM || most <= 1) throw;
@@ -412,31 +406,28 @@ void ensemble_plan(Batch &b, int NP, int split)
     }
 }
 
-// Times three stages per row width and item size, and keeps the fastest: one
-// stage alone overrates small items, which end evenly but cost more slabs.
-// Positions and velocities are not written: steps of length 0 would leave finite
-// ones as they are, but turn those of a particle whose force is infinite or NaN
-// into NaN.
+// Times three stages per item size, and keeps the fastest: one stage alone
+// overrates small items, which end evenly but cost more slabs. Positions and
+// velocities are not written: steps of length 0 would leave finite ones as they
+// are, but turn those of a particle whose force is infinite or NaN into NaN.
 void ensemble_tune(Batch &b)
 {
     Ctx &c = ctx();
-    static const int splits[] = {6, 16, 40};
     float best = 1e30f;
-    int bn = 2, bs = 16;
-    for (int np = 2; np <= 4; np += 2)
-        for (int sp : splits) {
-            ensemble_plan(b, np, sp);
-            ensemble_run(b, 0, 0.0, -1, true);  // warm
-            STEPS_CUDA(cudaEventRecord(c.marks[12], c.stream));
-            ensemble_run(b, 2, 0.0, -1, true);
-            STEPS_CUDA(cudaEventRecord(c.marks[13], c.stream));
-            STEPS_CUDA(cudaEventSynchronize(c.marks[13]));
-            float ms = 0;
-            STEPS_CUDA(cudaEventElapsedTime(&ms, c.marks[12], c.marks[13]));
-            if (ms < best) { best = ms; bn = np; bs = sp; }
-        }
+    int bs = 16;
+    for (int sp : {6, 16, 40}) {
+        ensemble_plan(b, sp);
+        ensemble_run(b, 0, 0.0, -1, true);  // warm
+        STEPS_CUDA(cudaEventRecord(c.marks[12], c.stream));
+        ensemble_run(b, 2, 0.0, -1, true);
+        STEPS_CUDA(cudaEventRecord(c.marks[13], c.stream));
+        STEPS_CUDA(cudaEventSynchronize(c.marks[13]));
+        float ms = 0;
+        STEPS_CUDA(cudaEventElapsedTime(&ms, c.marks[12], c.marks[13]));
+        if (ms < best) { best = ms; bs = sp; }
+    }
     check_kernel_status();
-    ensemble_plan(b, bn, bs);
+    ensemble_plan(b, bs);
     b.ens_tuned = true;
 }
 
@@ -628,7 +619,7 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
                 const int k = b.stall_rel;
                 b.stall_rel = -1;
                 if (!b.ens_tuned) ensemble_tune(b);
-                else ensemble_plan(b, b.ens_np, b.ens_split);
+                else ensemble_plan(b, b.ens_split);
                 release_graph(b);
                 ensemble_run(b, a.nsteps, a.h, k);
                 STEPS_CUDA(cudaStreamSynchronize(c.stream));
@@ -665,7 +656,7 @@ int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double
                 b.graph_guard != c.shape.guard) {
                 release_graph(b);
                 // the plan of the chosen path (the two paths keep their own shapes)
-                if (persistent) ensemble_plan(b, b.ens_np, b.ens_split);
+                if (persistent) ensemble_plan(b, b.ens_split);
                 else plan(b, b.threads_pp, b.ipt_pp);
                 if (!persistent) batch_forces(b);  // sizes every buffer before capture
                 kernel_status_word();              // allocated outside the capture

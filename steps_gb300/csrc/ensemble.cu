@@ -22,11 +22,19 @@
 // not depend on it). What other warps rewrite during the run (tile data,
 // positions, velocities, slabs) is read through L2.
 //
+// FP32 sums are half as long as in pair_sym.cu (SHORT in sym_r3.cuh), and rows
+// are 128 particles: against the one-sided kernel that this one replaced
+// (tiles of 128; 24 sets of 4,736 to 27,000 particles, relative errors against
+// FP64, median / 99th percentile: 2.55e-7 / 1.41e-6) the error was 4-7 % larger
+// with the longer sums and 16-22 % with rows of 256; it is 2.36e-7 / 1.37e-6.
+// The short sums cost 0.5 % (12 x 8,192 particles) to 1.5 % (3 x 20,000); rows
+// of 256 were the slower ones at every size tried (500 to 250,000).
+//
 // Measured (12 realisations of 4,736 to 65,024 particles, 1 + 4 stages, 6.4e10
-// ordered pairs): whole batch call with the data 35.2 ms with the one-sided
-// kernel that this one replaced, 27.7 with this one; 4.8 ms a stage, 2.7e12
-// pairs/s, of which the finish tasks are 3 %. Four blocks an SM, as in
-// pair_sym.cu: 24.1 ms for the run against 24.5 with 6 blocks for narrow rows.
+// ordered pairs): whole batch call with the data 34.9 ms with the one-sided
+// kernel, 27.8 with this one; 4.8 ms a stage, 2.7e12 pairs/s, of which the
+// finish tasks are 3 %. Four blocks an SM, as in pair_sym.cu: 24.1 ms for the run
+// against 24.5 with 6 blocks.
 #include <algorithm>
 
 #include "context.cuh"
@@ -150,7 +158,7 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
     for (int s = 0; s < R.C; s++)
 #pragma unroll
         for (int c = 0; c < 3; c++) f[c] += __ldcg(pi + ((size_t)s * 3 + c) * R.npad + q);
-    const int row = q / R.gran;
+    const int row = q / SYM_T;
     const int ng = row > 0 ? (row - 1) / R.G + 1 : 0;
 #pragma unroll 8
     for (int A = 0; A < ng; A++) {
@@ -186,10 +194,9 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
     if (lane == 0 && !(stage == 0 && k == e.stall_rel)) atomicAdd(e.fin_done + k, 1ull);
 }
 
-template <int NP>
 __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(EnsembleArgs e)
 {
-    __shared__ __align__(16) SymWarp<NP> shw[SYM_WARPS];
+    __shared__ __align__(16) SymWarp<ENS_NP> shw[SYM_WARPS];
     __shared__ SymArgs sha[SYM_WARPS];  // each warp's item, out of the pair loop's registers
     const int lane = threadIdx.x & 31;
     SymArgs &a = sha[threadIdx.x >> 5];
@@ -232,7 +239,7 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(Ensembl
                 a.eps = e.eps + q0;
                 a.idx = e.idx + q0;
                 a.njt = R.ntiles;
-                a.nrows = R.nrows;
+                a.nrows = R.ntiles;
                 a.G = R.G;
                 a.C = R.C;
                 a.step = R.step;
@@ -242,7 +249,7 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(Ensembl
                 a.guard2 = e.guard2;
             }
             __syncwarp();
-            sym_item<NP, true>(a, shw[threadIdx.x >> 5], d.y, d.z);
+            sym_item<ENS_NP, true, true>(a, shw[threadIdx.x >> 5], d.y, d.z);
             __threadfence();
             __syncwarp();
             if (lane == 0) atomicAdd(e.pair_done + k, 1ull);
@@ -252,19 +259,16 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_ensemble(Ensembl
 
 }  // namespace
 
-int ensemble_blocks(int NP)
+int ensemble_blocks()
 {
     int occ = 0;
-    if (NP == 4) STEPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble<4>, SYM_THREADS, 0));
-    else STEPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble<2>, SYM_THREADS, 0));
+    STEPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, SYM_THREADS, 0));
     return std::max(occ, 1);
 }
 
-void ensemble_launch(int NP, const EnsembleArgs &e, cudaStream_t st)
+void ensemble_launch(const EnsembleArgs &e, cudaStream_t st)
 {
-    const int grid = ctx().nsm * ensemble_blocks(NP);
-    if (NP == 4) k_ensemble<4><<<grid, SYM_THREADS, 0, st>>>(e);
-    else k_ensemble<2><<<grid, SYM_THREADS, 0, st>>>(e);
+    k_ensemble<<<ctx().nsm * ensemble_blocks(), SYM_THREADS, 0, st>>>(e);
     note_launch("k_ensemble");
 }
 

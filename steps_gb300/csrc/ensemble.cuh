@@ -7,12 +7,15 @@
 
 namespace steps {
 
-// One realisation: its tiles (padded to whole rows), the split of its pairs
-// (SymPlan) and its slabs of partial sums.
+constexpr int ENS_NP = 2;  // rows of 64 ENS_NP particles
+static_assert(64 * ENS_NP == SYM_T, "a row of the ensemble kernel is a tile");
+
+// One realisation: its tiles, the split of its pairs (SymPlan) and its slabs of
+// partial sums.
 struct EnsRel {
-    int tile0, ntiles;            // first tile of the batch arrays; tiles that hold particles
-    int nrows, G, C, step, gran;  // as in SymArgs / SymPlan
-    int npair;                    // pair tasks of a stage; finish tasks: 4 ntiles
+    int tile0, ntiles;  // first tile of the batch arrays; tiles (rows)
+    int G, C, step;     // as in SymArgs / SymPlan
+    int npair;          // pair tasks of a stage; finish tasks: 4 ntiles
     size_t npad;
     size_t part;                  // first double of its slabs
 };
@@ -40,8 +43,7 @@ struct EnsembleArgs {
     int stall_rel;          // test hook: this realisation's stage-0 tiles are never reported done (-1: none)
 };
 
-// Launches the kernel with rows of 64 NP particles (NP 2 or 4).
-void ensemble_launch(int NP, const EnsembleArgs &e, cudaStream_t st);
-int ensemble_blocks(int NP);  // resident blocks per SM
+void ensemble_launch(const EnsembleArgs &e, cudaStream_t st);
+int ensemble_blocks();  // resident blocks per SM
 
 }  // namespace steps

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(SYM_THREADS, SYM_R3_BLOCKS) k_sym_r3(SymArgs a
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= a.nitems) return;
         const int A = item / a.C;
-        sym_item<NP, false>(a, shw[threadIdx.x >> 5], A, item - A * a.C);
+        sym_item<NP, false, false>(a, shw[threadIdx.x >> 5], A, item - A * a.C);
     }
 }
 

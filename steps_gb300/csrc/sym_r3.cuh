@@ -21,12 +21,13 @@ template <int NP>
 struct SymWarp {
     double acc[3][2 * NP][32];  // FP64 i sums; each entry is its lane's own
     float4 q[64];               // 32 j particles, stored twice in a row
+    float jhalf[3][32];         // far path: j sums over the first half of a rotation, each its lane's own
     union {
         struct {
             float4 ql[64];  // near path: their residuals, softening lengths and ids
             float2 qe[64];
         };
-        float half[3][2 * NP][32];  // far path: i sums over the first half of a tile, each its lane's own
+        float half[3][2 * NP][32];  // far path: i sums over the tile's earlier j particles, each its lane's own
     };
 };
 
@@ -162,10 +163,21 @@ __device__ __forceinline__ void r3_slots(const SymArgs &a, SymWarp<NP> &sh, int 
         for (int c = 0; c < 3; c++) sh.acc[c][2 * h + k][lane] += (double)f[k][c];
 }
 
+// v added to two FP32 sums.
+__device__ __forceinline__ void add_half(f2 v, float &a, float &b)
+{
+    float lo, hi;
+    f2_unpack(v, lo, hi);
+    a += lo;
+    b += hi;
+}
+
 // Item (A, ch) of the R^3 pairwise kernel: the rows of group A against its chunk
 // ch, by one warp. COH: tile data through L2 (other warps of the same launch
-// rewrite it between the stages of an ensemble).
-template <int NP, bool COH>
+// rewrite it between the stages of an ensemble). SHORT: FP32 sums of at most 32
+// terms on either side before partial sums are added (else 64 on the i side and
+// 32 NP on the j side).
+template <int NP, bool COH, bool SHORT>
 __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int A, int ch)
 {
     constexpr unsigned BITS = (unsigned)((1ull << (8 * NP)) - 1), GROUP_BITS = 0x03030303u & BITS;
@@ -236,18 +248,24 @@ __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int 
             double *oj = pj + (qj - jlo);
             const bool firstrow = r == row0;
             float4 nq = ld_tile<COH>(a.pack + qj);
-            // FP32 sums run over 64 j particles, the two halves of a tile are
-            // added, and the tile's sum goes to FP64: as short as in the
-            // one-sided packed kernel, whose error this kernel stays below
-            // (over whole tiles the median error at n = 2^20 was 3 % above it).
+            // FP32 i sums run over 64 j particles (SHORT: 32), the parts of a tile are
+            // added in FP32, and the tile's sum goes to FP64 (in one sum over whole
+            // tiles the median error at n = 2^20 was 3 % above the one-sided
+            // kernel's).
 #pragma unroll 1
             for (int g = 0; g < 4; g++) {
-                if (g == 2)
+                if (SHORT ? g > 0 : g == 2)
 #pragma unroll
                     for (int h = 0; h < NP; h++) {
-                        f2_unpack(AX[h], sh.half[0][2 * h][lane], sh.half[0][2 * h + 1][lane]);
-                        f2_unpack(AY[h], sh.half[1][2 * h][lane], sh.half[1][2 * h + 1][lane]);
-                        f2_unpack(AZ[h], sh.half[2][2 * h][lane], sh.half[2][2 * h + 1][lane]);
+                        if (SHORT && g > 1) {
+                            add_half(AX[h], sh.half[0][2 * h][lane], sh.half[0][2 * h + 1][lane]);
+                            add_half(AY[h], sh.half[1][2 * h][lane], sh.half[1][2 * h + 1][lane]);
+                            add_half(AZ[h], sh.half[2][2 * h][lane], sh.half[2][2 * h + 1][lane]);
+                        } else {
+                            f2_unpack(AX[h], sh.half[0][2 * h][lane], sh.half[0][2 * h + 1][lane]);
+                            f2_unpack(AY[h], sh.half[1][2 * h][lane], sh.half[1][2 * h + 1][lane]);
+                            f2_unpack(AZ[h], sh.half[2][2 * h][lane], sh.half[2][2 * h + 1][lane]);
+                        }
                         AX[h] = AY[h] = AZ[h] = 0ull;
                     }
                 const float4 q0 = nq;
@@ -260,8 +278,7 @@ __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int 
                 sh.q[lane] = sh.q[32 + lane] = q0;
                 __syncwarp();
                 f2 JX = 0ull, JY = 0ull, JZ = 0ull;
-#pragma unroll 16
-                for (int s = 0; s < 32; s++) {
+                auto step = [&](int s) {
                     const float4 q = sh.q[lane + s];
                     const f2 qx = f2_bcast(q.x), qy = f2_bcast(q.y), qz = f2_bcast(q.z), qm = f2_bcast(q.w);
 #pragma unroll
@@ -283,16 +300,40 @@ __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int 
                     JX = f2_shfl(JX, nxt);
                     JY = f2_shfl(JY, nxt);
                     JZ = f2_shfl(JZ, nxt);
-                }
-                if (both) {
-                    float v[3][2];
-                    f2_unpack(JX, v[0][0], v[0][1]);
-                    f2_unpack(JY, v[1][0], v[1][1]);
-                    f2_unpack(JZ, v[2][0], v[2][1]);
+                };
+                auto jsum = [&](float *v) {
+                    float lo, hi;
+                    f2_unpack(JX, lo, hi);
+                    v[0] = lo + hi;
+                    f2_unpack(JY, lo, hi);
+                    v[1] = lo + hi;
+                    f2_unpack(JZ, lo, hi);
+                    v[2] = lo + hi;
+                };
+                float v[3];
+                if constexpr (SHORT) {
+#pragma unroll 1
+                    for (int s0 = 0; s0 < 32; s0 += 16) {
 #pragma unroll
-                    for (int c = 0; c < 3; c++)
-                        add_slab(oj + c * jlen + g * 32, (double)(v[c][0] + v[c][1]), firstrow);
+                        for (int s = 0; s < 16; s++) step(s0 + s);
+                        jsum(v);
+                        if (s0 == 0) {  // of j particle (lane + 16) mod 32
+#pragma unroll
+                            for (int c = 0; c < 3; c++) sh.jhalf[c][(lane + 16) & 31] = v[c];
+                            JX = JY = JZ = 0ull;
+                            __syncwarp();
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; c++) v[c] += sh.jhalf[c][lane];
+                } else {
+#pragma unroll 16
+                    for (int s = 0; s < 32; s++) step(s);
+                    jsum(v);
                 }
+                if (both)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) add_slab(oj + c * jlen + g * 32, (double)v[c], firstrow);
             }
 #pragma unroll
             for (int h = 0; h < NP; h++) {

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 import steps_gb300 as S
-from helpers import err_stats
+from helpers import err_stats, rel_err
 from steps_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +72,26 @@ def test_precision_guard_between_runs(engine, graph):
         assert np.array_equal(before, run(30.0))
     finally:
         engine.set_guard(30.0)
+
+
+def test_errors_as_one_sided(engine):
+    """FP32 sums over as few terms as in the packed one-sided kernel with tiles of 128, and so the same errors against
+    FP64: 122,000 particles give the median to 0.3 % and the 99th percentile to 1 % (1 sigma)."""
+    sets = [W.r3_compactified(n, 300.0, seed=n + k, displace=True) for n in (4736, 9000, 20000, 27000) for k in (1, 2)]
+    p = S.params(S.R3)
+    engine.batch_set([s.x for s in sets], [s.m for s in sets], [s.eps for s in sets])
+    engine.batch_run(p, S.MIXED, 0, 1e-3, graph=1)
+    pairwise, one = [], []
+    engine.set_variant(1)
+    engine.set_tuning(128, 1, 0)
+    try:
+        for k, s in enumerate(sets):
+            engine.set_particles(s.m, s.eps)
+            F64 = engine.forces(s.x, p, S.FP64)
+            pairwise.append(rel_err(engine.batch_get(k)[2], F64))
+            one.append(rel_err(engine.forces(s.x, p, S.MIXED), F64))
+    finally:
+        engine.set_variant(0)
+        engine.set_tuning(128, 2, 0)
+    a, b = (np.percentile(np.concatenate(e), [50, 99]) for e in (pairwise, one))
+    assert a[0] < 1.02 * b[0] and a[1] < 1.04 * b[1], (a, b)
