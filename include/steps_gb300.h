@@ -230,8 +230,8 @@ int steps_gpu_batch_set(int count, const int *n, const double *const *x, const d
  * each pair of particles once, or add up, kick, drift and re-tile 32 particles,
  * each stage of a realisation starting when its previous stage is done (bounded
  * waits: STEPS_E_TIMEOUT if one gives up); item size autotuned on the first run.
- * graph = 2 runs it as a CUDA graph of per-phase kernels (re-ordering every step); graph = 0 as
- * `count` separate plain launches per phase. */
+ * graph = 2 runs it as a CUDA graph of per-phase kernels (re-ordering every
+ * step); graph = 0 as `count` separate plain launches per phase. */
 int steps_gpu_batch_run(const steps_params *p, int precision, int nsteps, double h, int graph);
 
 /* Downloads realisation k's positions/velocities/forces (any may be NULL). */
@@ -335,6 +335,12 @@ int steps_gpu_test_stall_copy(long long tile_seq);
  * stage run out after about a second; the call returns STEPS_E_TIMEOUT and the
  * context stays usable. -1 cancels. One shot. */
 int steps_gpu_test_stall_ensemble(int realisation);
+
+/* Test hook: the following persistent runs (graph = 1) of the registered batch
+ * use items of about 1 / split (in [1, 1000]) of a resident warp's share of a
+ * stage, like one of the plans that the first run otherwise times. split = 0:
+ * timed again at the next run. */
+int steps_gpu_test_ensemble_plan(int split);
 
 /* Debug bounds checks. libsteps_gb300_check.so is the same library built with
  * -DSTEPS_CHECK: every kernel compares its tile, chunk, slot, output-row,

@@ -255,6 +255,9 @@ class Engine:
     def test_stall_ensemble(self, realisation: int):
         self._check(self.lib.steps_gpu_test_stall_ensemble(int(realisation)))
 
+    def test_ensemble_plan(self, split: int):
+        self._check(self.lib.steps_gpu_test_ensemble_plan(int(split)))
+
     def checks_compiled(self) -> bool:
         return bool(self.lib.steps_gpu_checks_compiled())
 

@@ -704,6 +704,27 @@ int steps_gpu_test_stall_ensemble(int realisation)
         &realisation);
 }
 
+int steps_gpu_test_ensemble_plan(int split)
+{
+    return run_guarded(
+        [](void *vp) {
+            const int split = *static_cast<int *>(vp);
+            require_init();
+            Batch *b = ctx().batch;
+            if (!b) fail(STEPS_E_STATE, "no batch: call steps_gpu_batch_set first");
+            if (split < 0 || split > 1000) fail(STEPS_E_ARG, "test_ensemble_plan: split must be in [0, 1000]");
+            release_graph(*b);
+            b->ens_tuned = false;
+            if (split == 0) return;
+            ensemble_plan(*b, split);
+            ensemble_run(*b, 0, 0.0, -1, true);  // sizes every buffer before a capture
+            STEPS_CUDA(cudaStreamSynchronize(ctx().stream));
+            check_kernel_status();
+            b->ens_tuned = true;
+        },
+        &split);
+}
+
 int steps_gpu_batch_get(int k, double *x, double *v, double *F)
 {
     struct A {

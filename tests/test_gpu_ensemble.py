@@ -95,3 +95,39 @@ def test_errors_as_one_sided(engine):
         engine.set_tuning(128, 2, 0)
     a, b = (np.percentile(np.concatenate(e), [50, 99]) for e in (pairwise, one))
     assert a[0] < 1.02 * b[0] and a[1] < 1.04 * b[1], (a, b)
+
+
+@pytest.mark.parametrize("split", [1, 6, 16, 40, 1000])
+def test_every_plan(engine, split):
+    """Each plan that the first run times (and a coarser and a finer one), whichever it would choose: realisations
+    below, at and above one tile, of one and of several tiles to a group, and 0 and 2 steps."""
+    sizes = (1, 2, 127, 128, 129, 257, 900, 5000, 20000)
+    sets = [W.r3_compactified(max(n, 2), 300.0, seed=n, displace=True) for n in sizes]
+    xs, ms, es = ([getattr(s, f)[:n] for s, n in zip(sets, sizes)] for f in ("x", "m", "eps"))
+    p, h = S.params(S.R3), 1e-3
+    for steps in (0, 2):
+        engine.batch_set(xs, ms, es)
+        engine.test_ensemble_plan(split)
+        engine.batch_run(p, S.MIXED, steps, h, graph=1)
+        got = [engine.batch_get(k) for k in range(len(sizes))]
+        for k, (x, v, F) in enumerate(got):
+            engine.set_particles(ms[k], es[k])
+            F64 = engine.forces(x, p, S.FP64)
+            if sizes[k] == 1:
+                assert not F.any() and not v.any() and np.array_equal(x, xs[k])
+                continue
+            assert err_stats(F, F64)["p99"] < 1e-5, (sizes[k], steps)
+            if steps == 0:
+                assert np.array_equal(x, xs[k]) and not v.any()
+                continue
+            engine.upload_positions(xs[k])
+            engine.upload_velocities(np.zeros_like(xs[k]))
+            engine.kdk(p, S.FP64, steps, h)
+            x64, v64, _ = engine.state()
+            assert np.abs(x - x64).max() < 1e-9 * (1 + np.abs(x64).max()), sizes[k]
+            assert err_stats(v, v64)["p99"] < 1e-5, sizes[k]
+    engine.test_ensemble_plan(0)
+    for bad in (-1, 1001):
+        with pytest.raises(S.StepsError) as e:
+            engine.test_ensemble_plan(bad)
+        assert e.value.code == S.STEPS_E_ARG
