@@ -46,7 +46,6 @@ struct Batch {
     DevBuf tslot;                 // int2 per tile: first partial slot, number of slots
     DevBuf part, counter, err;
     int T = 0, ntiles = 0, nitems = 0, threads = 0, ipt = 0, grid = 0;
-    int jmax = 256;  // j tiles per work item at most
     long long graph_kernels = 0;
     int nmax = 0;  // largest realisation
     bool tuned = false;     // per-phase graph shape
@@ -155,11 +154,10 @@ __global__ void k_batch_reduce(const double *__restrict__ part, const int2 *__re
 }
 
 // Tile descriptors and the work list for tile size T (host side, once per shape).
-void plan(Batch &b, int threads, int ipt, int jmax = 256)
+void plan(Batch &b, int threads, int ipt)
 {
     Ctx &c = ctx();
     const int T = threads * ipt;
-    b.jmax = jmax;
     std::vector<int> tstart(b.count), nt(b.count);
     std::vector<int2> desc;
     for (int k = 0; k < b.count; k++) {
@@ -168,14 +166,14 @@ void plan(Batch &b, int threads, int ipt, int jmax = 256)
         for (int t = 0; t < nt[k]; t++) desc.push_back(make_int2(b.off[k] + t * T, std::min(T, b.n[k] - t * T)));
     }
     b.ntiles = (int)desc.size();
-    // Items: per realisation i tiles x j chunks of at most jmax tiles; largest realisations first.
+    // Items: per realisation i tiles x j chunks of at most 256 tiles; largest realisations first.
     std::vector<int> order(b.count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int d) { return b.n[a] > b.n[d]; });
     std::vector<int4> items;
     std::vector<int2> tslot(b.ntiles);
     for (int k : order) {
-        const int S = div_up(nt[k], jmax);
+        const int S = div_up(nt[k], 256);
         const int per = div_up(nt[k], S);
         for (int I = 0; I < nt[k]; I++) {
             const int gI = tstart[k] + I;
@@ -315,7 +313,6 @@ void ensemble_run(Batch &b, int nsteps, double h, int stall_rel, bool hold = fal
     e.hold = hold;
     e.guard2 = c.shape.guard * c.shape.guard;
     e.n = b.ntot;
-    e.ntiles = b.ntiles;
     e.status = kernel_status_word();
     e.stall_rel = stall_rel;
     e.wait_cycles = (long long)(b.ens_wait * (double)mixed::MBAR_WAIT_CYCLES);

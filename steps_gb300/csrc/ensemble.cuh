@@ -37,7 +37,7 @@ struct EnsembleArgs {
     bool hold;              // stages are evaluated and tiles rebuilt, x and v left as they are (timing)
     double h;               // fixed step; acceleration g F a^-3 - 2 H v with g = 1, a = 1, H = 0
     float guard2;
-    int n, ntiles;
+    int n;                  // particles of all realisations (bounds checks)
     long long wait_cycles;  // SM clock cycles after which a wait gives up
     int *status;            // STEPS_E_TIMEOUT when a wait gave up
     int stall_rel;          // test hook: this realisation's stage-0 tiles are never reported done (-1: none)
