@@ -126,6 +126,14 @@ void DevBuf::grow(size_t want)
     bytes = sz;
 }
 
+bool DevBuf::fits(size_t want) const
+{
+    if (want <= bytes && p) return true;
+    size_t free_bytes = 0, total = 0;
+    STEPS_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    return want <= free_bytes + bytes;
+}
+
 void DevBuf::release()
 {
     if (p) cudaFree(p);

@@ -34,6 +34,10 @@ struct DevBuf {
     template <class T>
     T *ensure(size_t count) { grow(count * sizeof(T)); return static_cast<T *>(p); }
     void grow(size_t want);
+    // Whether the buffer holds `want` bytes, or could if it were released and
+    // allocated again: a call that has a way to do with less asks first, since a
+    // grow() that fails has released the old buffer.
+    bool fits(size_t want) const;
     void release();
 };
 

@@ -503,7 +503,8 @@ void forces_fp64(const KParams &kp, const Tables &tb, const double *x, int n, in
     int jchunk = div_up(div_up(n, S), FP64_THREADS) * FP64_THREADS;
     S = div_up(n, jchunk);
     SymPlan plan, *sym = nullptr;
-    if (id_min == 0 && ni == n && n >= SYM_FP64_MIN_N && fp64_odd(kp, tb) && fp64_plan(n, plan)) {
+    if (id_min == 0 && ni == n && n >= SYM_FP64_MIN_N && fp64_odd(kp, tb) && fp64_plan(n, plan) &&
+        c.partial.fits(plan.doubles * sizeof(double))) {
         try {
             c.partial.ensure<double>(plan.doubles);
             c.counter.ensure<unsigned>(4);

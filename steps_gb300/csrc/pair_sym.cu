@@ -176,8 +176,9 @@ void sym_reduce(const SymPlan &p, const double *part, const uint32_t *perm, int 
 bool sym_supported(const KParams &kp, const Tables &tb, int n)
 {
     SymPlan p;
-    if (kp.topology == STEPS_R3) return n >= SYM_MIN_N && sym_plan(n, p);
-    return n >= BOX_MIN_N && box_plan(n, p) && box_supported(kp, tb);
+    const bool ok = kp.topology == STEPS_R3 ? n >= SYM_MIN_N && sym_plan(n, p)
+                                            : n >= BOX_MIN_N && box_plan(n, p) && box_supported(kp, tb);
+    return ok && ctx().partial.fits(p.doubles * sizeof(double));
 }
 
 void forces_sym(const KParams &kp, const Tables &tb, const double *x, const double *m64, const double *eps64, int n,

@@ -296,3 +296,54 @@ def test_fp64_outside_the_fp32_range(fresh, port, scale, entry):
     Fo = port.forces(port.system(0, m, eps, port_params(O)), x)
     # FP64 sums of 600 terms: about 600 roundings of 1.1e-16 of the sum of magnitudes, which cancels to 1e-2 at worst
     assert rel_err(F, Fo).max() < 1e-11
+
+
+# ---- device memory ----------------------------------------------------------------
+
+
+@pytest.mark.parametrize("precision", [S.MIXED, S.FP64])
+@pytest.mark.parametrize("kind", ["r3", "s12"])
+def test_partial_sums_that_do_not_fit(fresh, kind, precision):
+    """Where the pairwise kernel's partial sums do not fit in device memory the call runs the one-sided kernel, with its
+    launches only (no attempt first) and its result; with the memory back it is pairwise again."""
+    torch = pytest.importorskip("torch")
+    n = 100000 if precision == S.MIXED else 30000
+    ps, p = (W.r3_compactified(n, 480.0, seed=2, displace=True), S.params(S.R3)) if kind == "r3" else periodic(fresh, kind, n)
+
+    def call(eng):
+        before = eng.launch_count()
+        F = eng.forces(ps.x, p, precision)
+        return F, eng.launch_count() - before
+
+    fresh.set_particles(ps.m, ps.eps)
+    if precision == S.MIXED:  # the one-sided shape of this size
+        if kind == "r3":
+            fresh.set_variant(1)
+        fresh.set_tuning(*((128, 2, 0) if kind == "r3" else (64, 1, 0)))
+        one, launches = call(fresh)
+    else:
+        one = np.concatenate([fresh.forces(ps.x, p, precision, 0, 0), fresh.forces(ps.x, p, precision, 1, n - 1)])
+        launches = 3
+    fresh.shutdown()
+    eng = S.Engine(0)
+    eng.set_particles(ps.m[:4000], ps.eps[:4000])
+    eng.forces(ps.x[:4000], p, precision)
+    eng.set_particles(ps.m, ps.eps)
+    torch.cuda.init()
+    # the slabs: 24 bytes for each particle, at least 128 + 128 of them on average
+    room = 24 * n * 150
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    try:
+        got = [call(eng) for _ in range(3)]
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    for F, count in got[1:]:  # the first call allocates what else it needs
+        if precision == S.MIXED:
+            assert np.array_equal(F, one)
+        else:
+            assert rel_err(F, one).max() < 1e-11
+        assert count == launches
+    F, count = call(eng)
+    assert not np.array_equal(F, got[0][0])
+    assert rel_err(F, one).max() < (1e-3 if precision == S.MIXED else 1e-11)
