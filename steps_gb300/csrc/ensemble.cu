@@ -159,7 +159,8 @@ __device__ __noinline__ void finish_block(const EnsembleArgs &e, int k, int b, i
 #pragma unroll
         for (int c = 0; c < 3; c++) f[c] += __ldcg(pi + ((size_t)s * 3 + c) * R.npad + q);
     const int row = q / SYM_T;
-    const int ng = row > 0 ? (row - 1) / R.G + 1 : 0;
+    int ng = row > 0 ? (row - 1) / R.G + 1 : 0;
+    STEPS_CHECK_IDX(ng, R.npair / R.C + 1, CK_SLOT);
 #pragma unroll 8
     for (int A = 0; A < ng; A++) {
         const size_t start = (size_t)A * R.step, len = R.npad - start;

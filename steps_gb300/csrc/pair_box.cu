@@ -426,6 +426,9 @@ __global__ void __launch_bounds__(SYM_THREADS, box_blocks(K)) k_sym_box(BoxArgs 
         const int I0 = b0 >> 2, tiles = a.s.njt - I0;
         const int J0 = I0 + (int)((long long)tiles * ch / a.s.C);
         const int J1 = I0 + (int)((long long)tiles * (ch + 1) / a.s.C);
+        if (!check_item(A, div_up(a.s.nrows, a.s.G), ch, a.s.C, 32LL * b0, 32LL * b1, (long long)J0 * SYM_T,
+                        (long long)J1 * SYM_T, a.s.step, a.s.tri, npad, (long long)a.s.njt * SYM_T))
+            continue;
         const size_t jlo = a.s.tri ? (size_t)I0 * SYM_T : 0, jlen = npad - jlo;
         double *pj = a.s.pj + 3 * sym_slab(A, a.s.step, a.s.tri, npad);
         double *pi = a.s.pi + (size_t)ch * 3 * npad;

@@ -346,6 +346,9 @@ __global__ void __launch_bounds__(FP64_THREADS) k_sym_fp64(SymFp64Args a, KParam
         const int r0 = A * a.G, r1 = min(a.nrows, r0 + a.G);
         const int J0 = r0 + (int)((long long)(a.nrows - r0) * ch / a.C);
         const int J1 = r0 + (int)((long long)(a.nrows - r0) * (ch + 1) / a.C);
+        if (!check_item(A, div_up(a.nrows, a.G), ch, a.C, 32LL * r0, 32LL * r1, 32LL * J0, 32LL * J1, a.step, a.tri, a.npad,
+                        (long long)a.npad))
+            continue;
         const size_t jlo = a.tri ? (size_t)r0 * 32 : 0, jlen = a.npad - jlo;
         double *pj = a.pj + 3 * sym_slab(A, a.step, a.tri, a.npad);
         for (int r = r0; r < r1; r++) {

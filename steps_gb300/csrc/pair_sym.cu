@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_sym_reduce(const double *__r
 #pragma unroll
         for (int c = 0; c < 3; c++) f[c] += pi[((size_t)s * 3 + c) * p.npad + q];
     const int r = q / p.gran;  // met from the i side by the granules before its own
-    const int ng = r > 0 ? (r - 1) / p.G + 1 : 0;
+    int ng = r > 0 ? (r - 1) / p.G + 1 : 0;
+    STEPS_CHECK_IDX(ng, p.groups + 1, CK_SLOT);
 #pragma unroll 4
     for (int A = w; A < ng; A += RED_PARTS) {
         const size_t start = p.tri ? (size_t)A * p.step : 0, len = p.npad - start;

@@ -761,12 +761,6 @@ __global__ void k_table_records(const double *__restrict__ t, int ng, int halo, 
 // need no per-pair wrap. It grows with the grid (cells shrink as L / ng, tile
 // extents do not): 16 cells at ng = 63, ng / 8 above 128.
 inline int t3_halo(int ng) { return ng / 8 > 16 ? ng / 8 : 16; }
-// Room for the stencil records: an even extent holds whole bricks.
-inline size_t t3_records(int ng)
-{
-    const size_t e = ((size_t)ng + 2 * t3_halo(ng) + 1) / 2 * 2;
-    return e * e * e;
-}
 
 // FP32 float4 haloed copy of the FP64 table, rebuilt whenever the table changes.
 const float4 *t3_table_f32(const Tables &tb, cudaStream_t st)
@@ -788,7 +782,7 @@ const float4 *t3_table_f32(const Tables &tb, cudaStream_t st)
 const float4 *t3_table_records(const Tables &tb, int order, cudaStream_t st)
 {
     Ctx &c = ctx();
-    const size_t nrec = t3_records(tb.t3_ng);
+    const size_t nrec = t3_records(tb.t3_ng + 2 * t3_halo(tb.t3_ng));
     if (c.t3r_version != c.t3_version || c.t3r_order != order || !c.t3r.p) {
         float4 *o = c.t3r.ensure<float4>(3 * nrec);  // 2 nrec xy records, then nrec z records
         const size_t ext = (size_t)tb.t3_ng + 2 * t3_halo(tb.t3_ng), ncell = ext * ext * ext;
@@ -815,7 +809,7 @@ void t3_args(MixedArgs &a, const KParams &kp, const Tables &tb, cudaStream_t st)
     if (kp.is_periodic >= 2) {
         a.t3f = t3_table_f32(tb, st);
         a.t3r = t3_table_records(tb, kp.order == 4 ? 4 : 2, st);
-        a.t3rz = a.t3r + 2 * t3_records(tb.t3_ng);
+        a.t3rz = a.t3r + 2 * t3_records(a.ext);
         a.ih = (float)((double)tb.t3_ng / kp.L);
         a.u0 = (float)((double)tb.t3_ng * 0.5 - 0.5);
     }

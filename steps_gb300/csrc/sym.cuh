@@ -47,6 +47,24 @@ __host__ __device__ inline size_t sym_slab(int A, int step, int tri, size_t npad
     return (size_t)A * npad - (tri ? (size_t)step * ((size_t)A * (A - 1) / 2) : 0);
 }
 
+// Bounds-checked builds: whether the padded particles [i0, i1) and [j0, j1) of
+// item (A, ch), the i slab ch and the words of the j slab A that it writes lie
+// in their arrays; the first that does not is recorded and the item is left out.
+__device__ __forceinline__ bool check_item(int A, int groups, int ch, int C, long long i0, long long i1, long long j0,
+                                           long long j1, int step, int tri, size_t npad, long long nj)
+{
+#ifdef STEPS_CHECK
+    const long long slab = 3 * (long long)sym_slab(A, step, tri, npad), end = 3 * (long long)sym_slab(A + 1, step, tri, npad);
+    const long long jlo = tri ? (long long)A * step : 0, jlen = (long long)npad - jlo;
+    return check_span(A, A, groups, CK_I_TILE) && check_span(ch, ch, C, CK_CHUNK) &&
+           (i0 >= i1 || check_span(i0, i1 - 1, (long long)npad, CK_I_TILE)) &&
+           (j0 >= j1 || (check_span(j0, j1 - 1, nj, CK_J_TILE) && check_span(j0 - jlo, j1 - 1 - jlo, jlen, CK_J_TILE) &&
+                         check_span(slab + j0 - jlo, slab + 2 * jlen + j1 - 1 - jlo, end, CK_SLOT)));
+#else
+    return true;
+#endif
+}
+
 // Adds to a partial sum that only this thread writes: the first contribution
 // is stored, later ones are added in the memory system, in program order, so
 // the sum is deterministic.

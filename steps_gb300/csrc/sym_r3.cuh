@@ -187,13 +187,16 @@ __device__ __forceinline__ void sym_item(const SymArgs &a, SymWarp<NP> &sh, int 
     const int J0 = first + (int)((long long)tiles * ch / a.C);
     const int J1 = first + (int)((long long)tiles * (ch + 1) / a.C);
 
+    if (!check_item(A, div_up(a.nrows, a.G), ch, a.C, (long long)row0 * NP * SYM_HALF, (long long)row1 * NP * SYM_HALF,
+                    (long long)J0 * SYM_T, (long long)J1 * SYM_T, a.step, 1, a.npad, (long long)a.njt * SYM_T))
+        return;
+
     // this group's j slab: the padded particles from its first tile on
     const size_t jlo = (size_t)first * SYM_T, jlen = a.npad - jlo;
     double *pj = a.pj + 3 * sym_slab(A, a.step, 1, a.npad);
 
     for (int r = row0; r < row1; r++) {
-        int H0 = r * NP;  // this row's half tiles: H0 .. H0 + NP - 1
-        STEPS_CHECK_IDX(H0, a.nrows * NP, CK_I_TILE);
+        const int H0 = r * NP;  // this row's half tiles: H0 .. H0 + NP - 1
         const int Ja = max(J0, H0 / 2);
 #pragma unroll
         for (int c = 0; c < 3; c++)

@@ -64,6 +64,13 @@ __host__ __device__ __forceinline__ int t3_record(int x, int y, int z, int E)
     return ((((x >> 1) * H + (y >> 1)) * H + (z >> 1)) << 3) + ((x & 1) << 2) + ((y & 1) << 1) + (z & 1);
 }
 
+// Room for the records of either order: an even extent holds whole bricks.
+__host__ __device__ __forceinline__ size_t t3_records(int E)
+{
+    const size_t e = ((size_t)E + 1) / 2 * 2;
+    return e * e * e;
+}
+
 // Two float4 of a 32-byte aligned record in one 256-bit load (sm_100+):
 // the L1 data path, which bounds the table kernels, sees one request per
 // record instead of two. The S1xR2 CIC and TSC records are 32 bytes: CIC
@@ -245,7 +252,8 @@ __device__ __forceinline__ void t3_correction(const MixedArgs &a, bool halo, flo
                 float rx = 0.0f, ry = 0.0f, rz = 0.0f;
 #pragma unroll
                 for (int bb = 0; bb < 4; bb++) {
-                    const int cr = t3_record<4>(bx + aa, by + bb, bz, E);
+                    int cr = t3_record<4>(bx + aa, by + bb, bz, E);
+                    STEPS_CHECK_IDX(cr, t3_records(E), CK_T3_CELL);
                     float4 vx, vy;
                     ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
                     const float4 vz = __ldg(a.t3rz + cr);
@@ -261,7 +269,8 @@ __device__ __forceinline__ void t3_correction(const MixedArgs &a, bool halo, flo
             const float q00 = wy[0] * wz[0], q01 = wy[0] * wz[1], q10 = wy[1] * wz[0], q11 = wy[1] * wz[1];
 #pragma unroll
             for (int aa = 0; aa < 2; aa++) {
-                const int cr = t3_record<2>(bx + aa, by, bz, E);
+                int cr = t3_record<2>(bx + aa, by, bz, E);
+                STEPS_CHECK_IDX(cr, t3_records(E), CK_T3_CELL);
                 float4 vx, vy;
                 ldg_v8(a.t3r + 2 * (size_t)cr, vx, vy);
                 const float4 vz = __ldg(a.t3rz + cr);
