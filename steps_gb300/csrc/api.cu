@@ -601,17 +601,25 @@ int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out)
             // times at 32,768, 1.38 times at 2^20; periodic: 1.1-1.8 times
             // at 5,000, about twice from 8,000 on), so nothing is timed; one
             // evaluation sizes the buffers.
-            const bool keep_sym = c.shape.sym;
-            c.shape.sym = true;
+            // A shape set before gives way, as it does to a timed one: other
+            // calls go by the shape rule.
+            const Shape keep = c.shape;
+            const bool keep_fixed = c.shape_fixed;
+            Shape rule;
+            rule.guard = keep.guard;
+            rule.t3_cells = keep.t3_cells;
+            c.shape = rule;
+            c.shape_fixed = false;
             try {
                 compute_forces(p, STEPS_MIXED, id_min, id_max, false);
             } catch (...) {
-                c.shape.sym = keep_sym;
+                c.shape = keep;
+                c.shape_fixed = keep_fixed;
                 throw;
             }
             c.F_ni = 0;
             c.F_valid = false;
-            const Shape other = c.shape_fixed ? c.shape : auto_shape(kp, c.n, c.n);
+            const Shape other = auto_shape(kp, c.n, c.n);
             if (out) { out[0] = other.threads; out[1] = other.ipt; out[2] = other.variant; }
             return;
         }

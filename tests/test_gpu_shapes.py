@@ -98,3 +98,25 @@ def test_tricubic_line(fresh, count):
     assert err_stats(F[-300:], fresh.forces(ps.x, p, S.FP64, n - 300, n - 1))["p99"] < 1e-5
     fresh.set_tuning(64 if count * n < 1e8 else 256, 1, 0)
     assert (F == fresh.forces(ps.x, p, S.MIXED, lo, n - 1)).all()
+
+
+@pytest.mark.parametrize("kind", ["r3", "t3"])
+def test_autotune_replaces_a_set_shape(fresh, kind):
+    """After steps_gpu_autotune an earlier explicit choice no longer counts, for the ranges of a call whose all-particle
+    form is not timed either."""
+    n = 24000
+    if kind == "t3":
+        ps, p = W.t3_clumpy(n, 100.0, 3), S.params(S.T3, is_periodic=2, L=100.0, rsim=50.0, ewald_order=2)
+        fresh.build_table_t3(31, 100.0, 0.02, 2.0, 0.3, 3.0, 6.0)
+    else:
+        ps, p = W.r3_compactified(n, 480.0, seed=4, displace=True), S.params(S.R3)
+    fresh.set_particles(ps.m, ps.eps)
+    want = fresh.forces(ps.x, p, S.MIXED), fresh.forces(ps.x, p, S.MIXED, 100, 9000)
+    fresh.set_variant(0)
+    fresh.set_tuning(64, 4 if kind == "r3" else 2, 3)  # T^3 has no 64 x 4
+    assert not (want[0] == fresh.forces(ps.x, p, S.MIXED)).all()
+    assert not (want[1] == fresh.forces(ps.x, p, S.MIXED, 100, 9000)).all()
+    fresh.upload_positions(ps.x)
+    fresh.autotune(p)
+    assert (want[0] == fresh.forces(ps.x, p, S.MIXED)).all()
+    assert (want[1] == fresh.forces(ps.x, p, S.MIXED, 100, 9000)).all()
