@@ -246,7 +246,11 @@ int steps_gpu_batch_get(int k, double *x, double *v, double *F);
  * without one, and after steps_gpu_autotune, calls for the forces of all
  * particles (from 20,000 on in R^3, 4,096 on in the periodic topologies) run a
  * kernel that evaluates each pair once for both particles; with a correction
- * table only if the table is odd in the separation, as the builders' are. */
+ * table only if the table is odd in the separation, as the builders' are, and
+ * only if its partial sums (6.4 GB at 2^20 particles, 16 GiB at most, kept until
+ * steps_gpu_shutdown) fit in device memory. An explicit choice, the values
+ * that were once the defaults (128, 2, 0 and variant 0) included, holds until
+ * steps_gpu_autotune or steps_gpu_shutdown. */
 int steps_gpu_set_tuning(int threads, int ipt, int jsplit);
 
 /* R^3 mixed-precision pair loop: 0 = scalar FP32 instructions, 1 = packed
@@ -281,8 +285,9 @@ int steps_gpu_set_precision_guard(double ratio);
  * of work (after one untimed launch); the three best are timed again on 96
  * waves (or the whole range when it is smaller). Calls over all particles that
  * run the kernel evaluating each pair once (steps_gpu_set_tuning) are faster
- * than with any of these shapes: nothing is timed for them, and out is the
- * shape that other calls use. Leaves no resident forces. */
+ * than with any of these shapes: nothing is timed for them, other calls go by
+ * the rule for their size again, and out is the rule's shape for one-sided calls
+ * of this size. Leaves no resident forces. */
 int steps_gpu_autotune(const steps_params *p, int id_min, int id_max, int *out);
 
 /* Number of kernels this library has launched since init. */

@@ -108,9 +108,19 @@ void forces_mixed(const KParams &kp, const Tables &tb, const double *x, const do
 // partial sums are better (whole evaluation, us: n = 16,384 215 against 233;
 // 20,000 300 against 303; 24,000 377 against 365; 28,000 480 against 441).
 constexpr int SYM_MIN_N = 20000;
+// FP64: twice as fast at the line, even around 1,500, where the one-sided grid
+// ends with a full wave (whole call, us, one-sided / pairwise, R^3: n = 512 151 /
+// 75, 800 156 / 84, 1,500 155 / 168, 2,000 209 / 207; tricubic 1,710 / 492, 1,710
+// / 493, 1,712 / 1,370, 2,957 / 1,646). Smaller sets would gain too (300: 152 /
+// 108); the line is the smallest size at which each mode is tested.
 constexpr int SYM_FP64_MIN_N = 512;
-constexpr int BOX_MIN_N = 4096;  // periodic topologies (n = 3,000 / 5,000, one-sided tuned -> pairwise, us: trilinear 189 /
-                               // 393 -> 175 / 251, CIC 66 / 143 -> 101 / 119, images 95 / 179 -> 99 / 132)
+// Periodic topologies, one line between the kinds' own (whole call, us, one-sided
+// / pairwise at n = 3,000, 4,096, 5,000): nearest image on T^3 108 / 141, 137 /
+// 147, 155 / 156; CIC 120 / 169, 156 / 180, 194 / 190; images 156 / 163, 191 / 180,
+// 236 / 194; TSC 190 / 184, 268 / 232, 368 / 280; trilinear 255 / 255, 342 / 245,
+// 433 / 318; tricubic 1,380 / 1,015, 2,100 / 1,284, 2,884 / 1,762; 31 images 541 /
+// 337, 837 / 379, 1,148 / 400.
+constexpr int BOX_MIN_N = 4096;
 constexpr int SYM_NP4_N = 100000;  // from here on rows of 256 particles instead of 128
 constexpr long long SYM_PARTIAL_BYTES = 16LL << 30;  // FP64 partial sums of both sides at most
 bool sym_supported(const KParams &kp, const Tables &tb, int n);

@@ -608,8 +608,8 @@ __global__ void __launch_bounds__(SYM_THREADS, box_blocks(K)) k_sym_box(BoxArgs 
 // magnitudes order as integers, NaN above all. A thread takes a cell and its
 // mirror at a time and a block ends with one atomic per word: the first call
 // after an upload waits for this kernel, and with two atomics per cell on the
-// same two words it took 2.6 ms at Ng = 127 and 21 ms at 255 (with the copy and the wait; now 0.04
-// and 0.22).
+// same two words it took 2.6 ms at Ng = 127 and 21 ms at 255 (with the copy and
+// the wait; now 0.04 and 0.22).
 constexpr int PARITY_THREADS = 256;
 __device__ __forceinline__ unsigned long long magnitude_bits(double v)
 {

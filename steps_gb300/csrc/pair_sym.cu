@@ -38,10 +38,12 @@
 //
 // Measured (GB300, clustered compactified sets, pair kernel, one-sided packed
 // kernel -> this one): n = 32,768: 628 (tuned 525) -> 416 us; 262,144:
-// 28.3 -> 19.0 ms; 2^20: 404 -> 293 ms, the FMA pipe 77 % busy.
+// 28.3 -> 19.0 ms; 2^20: 404 -> 291 ms, 16 instructions a pair at 77 % of the
+// measured FMA issue rate (counted by ncu at 131,072: pipe 70 % active, 5.1 ms).
 // Scalar instead of packed sums and a single rotated sum instead of two
 // measured within 3 % or slower: the FMA pipe with its operand reads is the
-// limit. 16 warps an SM with all the registers they want do better than more:
+// limit. 16 warps an SM with 128 registers a thread (NP = 2 fits, NP = 4 spills
+// 12 bytes) do better than more:
 // NP = 2, 6 blocks of 80 registers 433 us at n = 32,768 and 648 at 39,999, 5
 // blocks 422 and 624, 4 blocks 416 and 613 (3: 449 and 650). The rotation is
 // unrolled 16 times (8 / 16 / 32 times: NP = 2, n = 32,768 420 / 416 / 449 us;
