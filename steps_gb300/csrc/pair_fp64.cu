@@ -166,12 +166,10 @@ __device__ __forceinline__ void s1r2_interp_fp64(const double *__restrict__ T, i
         double sr = ur - (double)jr, sz = uz - (double)jz;
         double wr[3] = {0.5 * (0.5 - sr) * (0.5 - sr), 0.75 - sr * sr, 0.5 * (0.5 + sr) * (0.5 + sr)};
         double wz[3] = {0.5 * (0.5 - sz) * (0.5 - sz), 0.75 - sz * sz, 0.5 * (0.5 + sz) * (0.5 + sz)};
-        int ir[3] = {jr - 1, jr, jr + 1};
-        if (ir[0] < 0) ir[0] = 0;
-        if (ir[1] < 0) ir[1] = 0;
-        if (ir[1] > nrho - 1) ir[1] = nrho - 1;
-        if (ir[2] > nrho - 1) ir[2] = nrho - 1;
-        int izs[3] = {pos_mod(jz - 1, nz), pos_mod(jz, nz), pos_mod(jz + 1, nz)};
+        // a NaN separation converts to the lowest int: clamped before it is used
+        const int jc = min(max(jr, 0), nrho - 1), zc = pos_mod(jz, nz);
+        const int ir[3] = {max(jc - 1, 0), jc, min(jc + 1, nrho - 1)};
+        const int izs[3] = {zc > 0 ? zc - 1 : nz - 1, zc, zc < nz - 1 ? zc + 1 : 0};
 #pragma unroll
         for (int zr = 0; zr < 3; zr++) {
             double w0 = wr[0] * wz[zr], w1 = wr[1] * wz[zr], w2 = wr[2] * wz[zr];
