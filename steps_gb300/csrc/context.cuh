@@ -166,7 +166,7 @@ __device__ __forceinline__ void add_background(const Background &bg, const doubl
         double r = sqrt(xi[0] * xi[0] + xi[1] * xi[1]);
         int sz = bg.radial_size;
         double step = bg.rsim / (double)sz;
-        int i = (int)floor(r / bg.rsim * (sz - 1));
+        int i = max((int)floor(r / bg.rsim * (sz - 1)), 0);  // NaN converts to the lowest int
         double c = bg.radial[sz - 1];
         if (i < sz - 1) {
             STEPS_CHECK_IDX(i, sz - 1, CK_RADIAL);

@@ -1,5 +1,6 @@
 """The pairwise kernels, the ordering and the ensemble plans on the bounds-checked build: their items (rows, j tiles,
-slabs), table records and ordering indices at the sizes where groups, chunks, tiles and bricks end."""
+slabs), table records and ordering indices at the sizes where groups, chunks, tiles and bricks end, and with positions
+that are not finite."""
 import os
 import re
 import subprocess
@@ -24,6 +25,7 @@ CASES = [
     "tests/test_gpu_shapes.py::test_ordering_sizes",
     "tests/test_gpu_shapes.py::test_radix_ordering_sizes",
     "tests/test_gpu_ensemble.py::test_every_plan",
+    "tests/test_gpu_nonfinite.py",
 ]
 
 

@@ -53,3 +53,22 @@ def test_position(fresh, kind, value):
                 if not np.isfinite(value) and not (kind == "images" and axis == 2):  # there, no image is inside the cut
                     assert np.isnan(F[n // 3]).any() and np.isnan(part[5]).any()
             assert np.array_equal(before, fresh.forces(ps.x, p, precision))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 1e300])
+def test_cylindrical_background(fresh, value):
+    """The radial-force table of a comoving S^1 x R^2 run is read at the particle's own radius."""
+    n = 700
+    ps = W.s1r2_cylindrical(n, LZ, 600.0, 1)
+    fresh.build_radial_table(1000, 600.0, LZ, 1000)
+    fresh.set_particles(ps.m, ps.eps)
+    p = S.params(S.S1R2, is_periodic=2, L=LZ, rsim=600.0, s1r2_images=1, cosmology=1, comoving=1, mius=1e-3)
+    for precision in (S.MIXED, S.FP64):
+        before = fresh.forces(ps.x, p, precision)
+        for axis in (0, 1):
+            x = ps.x.copy()
+            x[n // 3, axis] = value
+            F = fresh.forces(x, p, precision)
+            if not np.isfinite(value):
+                assert np.isnan(F[n // 3]).any()
+        assert np.array_equal(before, fresh.forces(ps.x, p, precision))
